@@ -5,7 +5,11 @@
 //
 // Upstream builds the Wigner-d planes degree by degree with Risbo's recursion
 // (s2fft/recursions/risbo.py:4-120), so every degree waits for the whole previous plane.
-// Here every entry (m, n) follows its own three-term recurrence in the degree
+// Here each (l, m) walks along n by its own three-term recurrence, fused with the sum over n
+// (rotate_walk_kernel). All arithmetic is double.
+//
+// The planes (generate_rotate_dls) are written once per entry, so there every (m, n) follows
+// its three-term recurrence in the degree, whose stores are consecutive in n
 // (Varshalovich, Moskalev & Khersonskii, Quantum Theory of Angular Momentum, sec. 4.8;
 // Kostelec & Rockmore, J. Fourier Anal. Appl. 14 (2008) 145-179):
 //   d^{l+1}_{mn} = U_l(m) R_l(n) [ (cos beta - m n q_l) d^l_{mn} - V_l(m) P_l(n) d^{l-1}_{mn} ],
@@ -14,49 +18,34 @@
 // started at l0 = max(|m|, |n|) from E[l0][a] = d^{l0}_{l0,a} = (-1)^{l0-a}
 // sqrt(binom(2 l0, l0+a)) c^{l0+a} s^{l0-a} (c = cos(beta/2), s = sin(beta/2)) through
 // d_{m,n} = (-1)^{m-n} d_{n,m} = d_{-n,-m}. Orders m < 0 follow from
-// d_{-m,-n} = (-1)^{m-n} d_{m,n}, so only m >= 0 is recurred. In double precision the
-// recurrence matches Risbo's planes to rounding (against a long-double run at L = 256:
-// 1e-15..8e-14 here, 1e-13..2e-13 for Risbo).
+// d_{-m,-n} = (-1)^{m-n} d_{m,n}, so only m >= 0 is recurred.
 //
-// Start values below 2^-960 are carried as a mantissa times 2^k (an int k < 0 per
+// Start values below 2^-960 are carried there as a mantissa times 2^k (an int k < 0 per
 // entry), renormalised in steps of 2^64 as they grow, and weighted by 2^k where they
 // contribute. The start table is the exponent-tracked product W = E^2,
 //   W_l = W_{l-1} 2l(2l-1) / ((l+a)(l-a)) (cs)^2,  W_{|a|} = c^{4a} (a >= 0), s^{4|a|} (a < 0),
 // formed in segments of 32 degrees with a carry pass, so no log-gamma enters.
-//
-// Schedule: a cluster of CTAs owns MT orders m0..m0+MT-1 (with their negatives) and all
-// n; lanes run along n in zigzag order (0, -1, 1, -2, ...) dealt to the cluster's CTAs
-// and warps in turn, so short and long n are shared alike. Each lane carries MT x S
-// recurrences in registers and walks l from m0 to L-1; its operands (T[l][|n|],
-// flm[l][+-n]) arrive through a cp.async ring in shared memory a few degrees ahead. Per
-// degree a warp reduces its 4 MT sums (+-m, re / im) by halving shuffles into shared
-// memory. Every kRotChunk degrees a CTA sums its warps and publishes the result with a
-// cluster arrive; after the matching wait, at the end of the next chunk, each CTA sums its
-// share of the outputs over the cluster's CTAs through distributed shared memory in rank
-// order (deterministic, no atomics) and writes them with exp(-i m alpha). With 8 orders
-// per tile and one n per lane (rotate_mma_kernel; clusters of up to 16 CTAs up to
-// L = 2048) the sum over a warp's 32 n runs on the FP64 tensor cores instead of shuffles.
-// The planes path writes every entry of [L][2L-1][2L-1] once, zeros included. All
-// arithmetic is double.
-#include <cooperative_groups.h>
+// A lane carries MT x S recurrences (MT orders, S values of n) in registers and walks l from
+// m0 to L-1; its operand T[l][|n|] arrives through a cp.async ring in shared memory a few
+// degrees ahead. Every entry of [L][2L-1][2L-1] is written once, zeros included.
 #include <cuda_runtime.h>
+#include <math_constants.h>
 
 #include <cmath>
 #include <cstdint>
 #include <type_traits>
+#include <utility>
 
 #include "s2b.h"
 #include "s2b_dev.h"
 #include "s2b_internal.h"
 #include "s2b_rotation.h"
 
-namespace cg = cooperative_groups;
-
 namespace s2b {
 namespace {
 
 constexpr int kRotSeg = 32;    // degrees per segment of the start-table product
-constexpr int kRotChunk = 16;  // degrees between cluster reductions
+constexpr int kRotChunk = 16;  // degrees of a staged coefficient chunk
 
 template <typename R2>
 struct RotIO;
@@ -89,19 +78,6 @@ __device__ __forceinline__ double warp_sum(double v) {
 // ---------------------------------------------------------------------------------
 // tables
 // ---------------------------------------------------------------------------------
-
-// exp(-i m alpha), exp(-i n gamma), m, n in [-(L-1), L-1]
-__global__ void rotate_phase_kernel(RotParams p) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * p.L - 1;
-       i += gridDim.x * blockDim.x) {
-    const double k = (double)(i - (p.L - 1));
-    double s, c;
-    sincos(-k * p.alpha, &s, &c);
-    p.ea[i] = make_double2(c, s);
-    sincos(-k * p.gamma, &s, &c);
-    p.eg[i] = make_double2(c, s);
-  }
-}
 
 // recurrence coefficients T and UVQ (beta-independent)
 __global__ void rotate_coef_kernel(RotParams p) {
@@ -236,70 +212,6 @@ __device__ __forceinline__ double pow2k(int k) {
   return k < -1022 ? 0.0 : __hiloint2double((k + 1023) << 20, 0);
 }
 
-// x[0..V-1] summed over the warp when slot s of lane holds value s ^ mask(lane),
-// mask = (lane >> (5 - log2 V)) & (V - 1): the halving exchanges need no selects, and
-// every lane ends with the total of value mask(lane)
-template <int V>
-__device__ __forceinline__ double reduce_perm(double* x) {
-#pragma unroll
-  for (int n = V, o = 16; n > 1; n >>= 1, o >>= 1) {
-#pragma unroll
-    for (int i = 0; i < n / 2; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i + n / 2], o);
-  }
-  double r = x[0];
-#pragma unroll
-  for (int o = 16 / V; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-  return r;
-}
-
-// split cluster barrier: arrive publishes this thread's earlier shared-memory writes to
-// the cluster, wait returns once every thread of the cluster has arrived
-__device__ __forceinline__ void cluster_arrive() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-
-// the cluster's sums of one chunk (cpart slot cp of every CTA, in rank order) phased and
-// written to out[b][l_first .. l_first + lc]; CTA `rank` takes every nr-th output
-template <typename R2, int MT>
-__device__ __forceinline__ void rotate_flush(const RotParams& p, const double* cp, int b,
-                                             int l_first, int lc, int m0, int rank) {
-  const int L = p.L, NN = 2 * L - 1, nr = p.nr, nt = blockDim.x;
-  cg::cluster_group cl = cg::this_cluster();
-  const int nout = (lc + 1) * 2 * MT;
-  for (int o = rank + nr * (int)threadIdx.x; o < nout; o += nr * nt) {
-    const int lco = o / (2 * MT), ci = o % (2 * MT), i = ci >> 1, sg = ci & 1;
-    const int m = m0 + i;
-    if (m >= L || (m == 0 && sg)) continue;
-    const int off = lco * 4 * MT + 4 * i + 2 * sg;
-    double re = 0.0, im = 0.0;
-#pragma unroll 1
-    for (int q0 = 0; q0 < nr; q0 += 4) {  // four remote loads in flight
-      double2 t[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        t[q] = q0 + q < nr ? *reinterpret_cast<const double2*>(
-                                 cl.map_shared_rank(const_cast<double*>(cp), q0 + q) + off)
-                           : make_double2(0.0, 0.0);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        re += t[q].x;
-        im += t[q].y;
-      }
-    }
-    if (sg && (m & 1)) {  // (-1)^m of the order -m
-      re = -re;
-      im = -im;
-    }
-    const int mo = sg ? -m : m;
-    const double2 a = p.ea[L - 1 + mo];
-    RotIO<R2>::put(p.out, ((size_t)b * L + l_first + lco) * NN + L - 1 + mo,
-                   make_double2(re * a.x - im * a.y, re * a.y + im * a.x));
-  }
-}
-
 // coefficients UVQ[l][m0 + i] of kRotChunk degrees from l0 into uvq[lc][i] (cp.async)
 template <int MT>
 __device__ __forceinline__ void rotate_stage(const RotParams& p, double4* uvq, int l0, int m0) {
@@ -316,24 +228,14 @@ constexpr int rot_depth() {  // degrees of the per-lane copy pipeline
   return S == 1 ? 4 : S == 2 ? 3 : 2;
 }
 
-// One cluster of p.nr CTAs (rank blockIdx.x) owns the orders m0 = MT blockIdx.y ..
+// The planes kernel. p.nr CTAs (rank blockIdx.x) own the orders m0 = MT blockIdx.y ..
 // m0 + MT - 1. Dynamic shared memory:
-//   ring  [D][S][3][blockDim] 16-byte slots: T[l][|n|], flm[l][n], flm[l][-n] of each lane,
-//         copied D - 1 degrees ahead
+//   ring  [D][S][blockDim] double2: T[l][|n|] of each lane, copied D - 1 degrees ahead
 //   uvq   [2][kRotChunk][MT] double4 coefficients, staged a chunk ahead
-//   (contraction) sbuf [kRotChunk][nw][4 MT] per-warp sums, cpart [3][kRotChunk][4 MT]
-//         per-CTA sums read by the cluster
-// Chunk k's CTA sums are published by a cluster arrive at its end and read after the
-// matching wait at the end of chunk k + 1, so CTAs run up to a chunk apart; three cpart
-// slots keep a slot unwritten until every CTA has read it.
-template <typename R2, int MT, int S, bool PL>
+template <int MT, int S>
 __global__ void __launch_bounds__(kRotThreads, 2) rotate_lrec_kernel(RotParams p) {
   extern __shared__ double4 smem4[];
-  constexpr int MG = MT < 4 ? MT : 4;  // orders per reduction group
-  constexpr int V = 4 * MG;            // sums per group: +m re, +m im, -m re, -m im per order
-  constexpr int LV = V == 8 ? 3 : 4;   // log2 V
   constexpr int D = rot_depth<S>();
-  constexpr bool contract = !PL;       // PL: planes only (generate_rotate_dls)
   static_assert(MT % 2 == 0, "tiles start at even orders");
   const int L = p.L, NN = 2 * L - 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nt = blockDim.x;
@@ -341,39 +243,24 @@ __global__ void __launch_bounds__(kRotThreads, 2) rotate_lrec_kernel(RotParams p
   const int m0 = blockIdx.y * MT;
   double* const dl = p.dl_out;
   double2* const ring = reinterpret_cast<double2*>(smem4);
-  double4* const uvq = smem4 + (D * S * 3 * nt) / 2;
-  double* const sbuf = reinterpret_cast<double*>(uvq + 2 * kRotChunk * MT);
-  double* const cpart = sbuf + kRotChunk * nw * 4 * MT;
+  double4* const uvq = smem4 + (D * S * nt) / 2;
 
-  // lane permutation of the reduction: slot s of a group holds sum s ^ mask, i.e. state
-  // slot is holds order is ^ pm within the group and sum slot c holds component c ^ cm
-  const int mask = contract ? (lane >> (5 - LV)) & (V - 1) : 0;
-  const int pm = mask >> 2, cm = mask & 3;
-
-  // this lane's n, one per S: the contraction deals n in zigzag order (j -> 0, -1, 1, -2,
-  // 2, ...) so that every warp slot holds short and long n alike; the planes take n in
-  // natural order (j -> j - (L-1)), so that a warp's stores cover 32 consecutive columns
+  // this lane's n, one per S, in natural order (j -> j - (L-1)), so that a warp's stores
+  // cover 32 consecutive columns
   int nv[S], an[S], wmin[S], wmax[S];
   double nd[S];
-  double2 eph[S];
 #pragma unroll
   for (int s = 0; s < S; ++s) {
-    const int gw = (s * nw + warp) * nr + rank;  // warp slot in the cluster's n order
+    const int gw = (s * nw + warp) * nr + rank;  // warp slot in the order of n
     const int j = gw * 32 + lane;
-    const int n = PL ? j - (L - 1) : (j & 1) ? -((j + 1) >> 1) : (j >> 1);
     const bool ok = j < NN;
-    nv[s] = ok ? n : 0;
+    nv[s] = ok ? j - (L - 1) : 0;
     nd[s] = (double)nv[s];
-    an[s] = ok ? abs(n) : L;  // L: never starts
-    if constexpr (PL) {  // least and largest |n| of the warp slot's (valid) n
-      const int lo = gw * 32 - (L - 1), hi = min(lo + 31, L - 1);
-      wmin[s] = (lo <= 0 && hi >= 0) ? 0 : min(abs(lo), abs(hi));
-      wmax[s] = max(abs(lo), abs(hi));
-    } else {
-      wmin[s] = 16 * gw;
-      wmax[s] = 16 * gw + 16;
-    }
-    eph[s] = ok && contract ? p.eg[L - 1 + n] : make_double2(0.0, 0.0);
+    an[s] = ok ? abs(nv[s]) : L;  // L: never starts
+    // least and largest |n| of the warp slot's (valid) n
+    const int lo = gw * 32 - (L - 1), hi = min(lo + 31, L - 1);
+    wmin[s] = (lo <= 0 && hi >= 0) ? 0 : min(abs(lo), abs(hi));
+    wmax[s] = max(abs(lo), abs(hi));
   }
   // degrees at which some entry of the warp slot starts: max(m, |n|) over its orders and lanes
   int wlo[S], whi[S], wany = wmin[0];  // wany: least |n| of the warp
@@ -384,553 +271,565 @@ __global__ void __launch_bounds__(kRotThreads, 2) rotate_lrec_kernel(RotParams p
     wany = min(wany, wmin[s]);
   }
 
-  const int nmaps = contract ? p.batch : 1;
-  int ck = 0;                          // chunks completed (all maps)
-  int pb = 0, plf = 0, plc = 0;        // the pending chunk: map, first degree, last index
+  // degrees below m0: the tile's rows are zero there
 #pragma unroll 1
-  for (int b = 0; b < nmaps; ++b) {
-    // degrees below m0: the tile's rows are zero there
-    if constexpr (contract) {
-      const int tot = m0 * 2 * MT;
-#pragma unroll 1
-      for (int e = rank * nt + tid; e < tot; e += nr * nt) {
-        const int l = e / (2 * MT), ci = e % (2 * MT), m = m0 + (ci >> 1);
-        if (m >= L || (m == 0 && (ci & 1))) continue;
-        RotIO<R2>::put(p.out, ((size_t)b * L + l) * NN + L - 1 + ((ci & 1) ? -m : m),
-                       make_double2(0.0, 0.0));
+  for (int l = 0; l < m0; ++l)
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      if (an[s] >= L) continue;
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const int m = m0 + i;
+        if (m >= L) continue;
+        dl[((size_t)l * NN + L - 1 + m) * NN + L - 1 + nv[s]] = 0.0;
+        if (m > 0) dl[((size_t)l * NN + L - 1 - m) * NN + L - 1 - nv[s]] = 0.0;
       }
-    } else {
+    }
+  // copies of consecutive degrees ll = m0, m0 + 1, ... into ring stage st (zero where
+  // nothing has started); with one n per lane the source pointer advances by one row
+  // per call, with more they are recomputed (fewer live registers)
+  const unsigned rbase = (unsigned)__cvta_generic_to_shared(ring + tid);
+  const double2* tq = p.T + (size_t)m0 * L + min(an[0], L - 1);
+  int ll = m0;
+  auto issue = [&](int st) {
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      const bool vt = ll < L && ll >= wmin[s];
+      const int lt = min(ll, L - 1);
+      const double2* ts = S == 1 ? tq : p.T + (size_t)lt * L + min(an[s], L - 1);
+      cp_async<16>(rbase + (unsigned)((st * S + s) * nt) * 16u, ts, vt);
+    }
+    if (S == 1 && ll + 1 < L) tq += L;
+    ++ll;
+  };
+  rotate_stage<MT>(p, uvq, m0, m0);
+  cp_async_commit();
+#pragma unroll
+  for (int k = 0; k < D - 1; ++k) {
+    issue(k);
+    cp_async_commit();
+  }
+  cp_async_wait<D - 1>();  // the coefficients of the first chunk
+  __syncthreads();
+
+  double v[MT][S], vp[MT][S];
+  int kx[MT][S];
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      v[i][s] = 0.0;
+      vp[i][s] = 0.0;
+      kx[i][s] = 0;
+    }
+  // some lane of the warp carries a start value below 2^-960 (kx < 0): warp-uniform
+  bool scaled = false;
+  int lc = 0, ub = 0, rs = 0;  // degree in chunk, coefficient buffer, ring stage
 #pragma unroll 1
-      for (int l = 0; l < m0; ++l)
+  for (int l = m0; l < L; ++l) {
+    const bool step = l + 1 < L;
+    // copies D - 1 degrees ahead, and the next chunk's coefficients at a chunk start
+    issue(rs == 0 ? D - 1 : rs - 1);  // degree l + D - 1
+    if (lc == 0 && l + kRotChunk < L)
+      rotate_stage<MT>(p, uvq + (ub ^ 1) * kRotChunk * MT, l + kRotChunk, m0);
+    cp_async_commit();
+    cp_async_wait<D - 1>();  // this degree's copies (this thread's own)
+    double2 tn[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) tn[s] = ring[(rs * S + s) * nt + tid];
+    rs = rs == D - 1 ? 0 : rs + 1;
+    const double4* const uvl = uvq + (ub * kRotChunk + lc) * MT;
+
+    // entries starting at this degree (only inside the warp slot's start window)
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      if (l < wlo[s] || l > whi[s]) continue;
+      bool neg = false;
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const int m = m0 + i;
+        if (l == max(m, an[s])) {  // E[l][col] (symmetries of d)
+          int col;
+          bool flip = false;
+          if (m >= an[s]) {
+            col = nv[s];
+          } else if (nv[s] > 0) {
+            col = m;
+            flip = ((m - nv[s]) & 1) != 0;
+          } else {
+            col = -m;
+          }
+          const RotXD e0 = p.start[(size_t)l * NN + L - 1 + col];
+          v[i][s] = flip ? -e0.m : e0.m;
+          kx[i][s] = e0.e;
+          vp[i][s] = 0.0;
+        }
+        neg |= kx[i][s] < 0;
+      }
+      scaled = __any_sync(0xffffffffu, neg) || scaled;
+    }
+    // warp slots not started yet: their entries of the planes are 0
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      if (l >= wmin[s] || an[s] >= L) continue;
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const int m = m0 + i;
+        if (m >= L) continue;
+        dl[((size_t)l * NN + L - 1 + m) * NN + L - 1 + nv[s]] = 0.0;
+        if (m > 0) dl[((size_t)l * NN + L - 1 - m) * NN + L - 1 - nv[s]] = 0.0;
+      }
+    }
+
+    // one degree of every started entry, branch-free so that the MT x S recurrences
+    // interleave; SC: with the 2^kx weights and the renormalisation
+    auto advance = [&](auto sc_tag) {
+      constexpr bool SC = decltype(sc_tag)::value;
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const double4 uv = uvl[i];
 #pragma unroll
         for (int s = 0; s < S; ++s) {
-          if (an[s] >= L) continue;
-#pragma unroll
-          for (int i = 0; i < MT; ++i) {
-            const int m = m0 + i;
-            if (m >= L) continue;
-            dl[((size_t)l * NN + L - 1 + m) * NN + L - 1 + nv[s]] = 0.0;
-            if (m > 0) dl[((size_t)l * NN + L - 1 - m) * NN + L - 1 - nv[s]] = 0.0;
+          if (S > 1 && l < wmin[s]) continue;  // warp-uniform
+          double dv = v[i][s];
+          if constexpr (SC) dv *= pow2k(kx[i][s]);
+          const int m = m0 + i;
+          if (an[s] < L && m < L) {
+            dl[((size_t)l * NN + L - 1 + m) * NN + L - 1 + nv[s]] = dv;
+            if (m > 0)
+              dl[((size_t)l * NN + L - 1 - m) * NN + L - 1 - nv[s]] =
+                  ((m - nv[s]) & 1) ? -dv : dv;
           }
-        }
-    }
-    const R2* const fb =
-        contract ? reinterpret_cast<const R2*>(p.flm) + (size_t)b * L * NN + L - 1 : nullptr;
-    // copies of consecutive degrees ll = m0, m0 + 1, ... into ring stage st (zero where
-    // nothing has started); with one n per lane the source pointers advance by one row
-    // per call, with more they are recomputed (fewer live registers)
-    const unsigned rbase = (unsigned)__cvta_generic_to_shared(ring + tid);
-    const double2* tq = p.T + (size_t)m0 * L + min(an[0], L - 1);
-    const R2* fq = contract ? fb + (size_t)m0 * NN + nv[0] : nullptr;
-    int ll = m0;
-    auto issue = [&](int st) {
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const bool vt = ll < L && ll >= wmin[s];
-        const unsigned r = rbase + (unsigned)(((st * S + s) * 3) * nt) * 16u;
-        const int lt = min(ll, L - 1);
-        const double2* ts = S == 1 ? tq : p.T + (size_t)lt * L + min(an[s], L - 1);
-        const R2* fs = S == 1 ? fq : fb + (size_t)lt * NN + nv[s];
-        cp_async<16>(r, ts, vt);
-        if constexpr (contract) {
-          const bool vf = vt && an[s] <= ll;
-          cp_async<sizeof(R2)>(r + 16u * nt, fs, vf);
-          cp_async<sizeof(R2)>(r + 32u * nt, fs - 2 * nv[s], vf);
-        }
-      }
-      if (S == 1 && ll + 1 < L) {
-        tq += L;
-        if constexpr (contract) fq += NN;
-      }
-      ++ll;
-    };
-    rotate_stage<MT>(p, uvq, m0, m0);
-    cp_async_commit();
-#pragma unroll
-    for (int k = 0; k < D - 1; ++k) {
-      issue(k);
-      cp_async_commit();
-    }
-    cp_async_wait<D - 1>();  // the coefficients of the first chunk
-    __syncthreads();
-
-    double v[MT][S], vp[MT][S];
-    int kx[MT][S];
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        v[i][s] = 0.0;
-        vp[i][s] = 0.0;
-        kx[i][s] = 0;
-      }
-    // some lane of the warp carries a start value below 2^-960 (kx < 0): warp-uniform
-    bool scaled = false;
-    int lc = 0, ub = 0, rs = 0;  // degree in chunk, coefficient buffer, ring stage
-#pragma unroll 1
-    for (int l = m0; l < L; ++l) {
-      const bool step = l + 1 < L;
-      // copies D - 1 degrees ahead, and the next chunk's coefficients at a chunk start
-      issue(rs == 0 ? D - 1 : rs - 1);  // degree l + D - 1
-      if (lc == 0 && l + kRotChunk < L)
-        rotate_stage<MT>(p, uvq + (ub ^ 1) * kRotChunk * MT, l + kRotChunk, m0);
-      cp_async_commit();
-      cp_async_wait<D - 1>();  // this degree's copies (this thread's own)
-      double2 tn[S], xa[S], xb[S];
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const double2* r = ring + ((rs * S + s) * 3) * nt + tid;
-        tn[s] = r[0];
-        if constexpr (contract) {
-          if constexpr (sizeof(R2) == 16) {
-            xa[s] = r[nt];
-            xb[s] = r[2 * nt];
-          } else {
-            const float2 fa = *reinterpret_cast<const float2*>(r + nt);
-            const float2 fc = *reinterpret_cast<const float2*>(r + 2 * nt);
-            xa[s] = make_double2(fa.x, fa.y);
-            xb[s] = make_double2(fc.x, fc.y);
+          if (step) {
+            const double t = fma(uv.z, nd[s], p.cb);
+            double vn = (uv.x * tn[s].x) * fma(t, v[i][s], -(uv.y * tn[s].y) * vp[i][s]);
+            double vc = v[i][s];
+            if constexpr (SC) {  // renormalise by up to 2^64 once |vn| >= 2^65
+              const bool big =
+                  kx[i][s] < 0 && (__double2hiint(vn) & 0x7ff00000) > ((1023 + 64) << 20);
+              const int sh = big ? min(64, -kx[i][s]) : 0;
+              const double f = __hiloint2double((1023 - sh) << 20, 0);
+              vn *= f;
+              vc *= f;
+              kx[i][s] += sh;
+            }
+            vp[i][s] = vc;
+            v[i][s] = vn;
           }
         }
       }
-      rs = rs == D - 1 ? 0 : rs + 1;
-      const double4* const uvl = uvq + (ub * kRotChunk + lc) * MT;
-
-      // entries starting at this degree (only inside the warp slot's start window)
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        if (l < wlo[s] || l > whi[s]) continue;
+      if constexpr (SC) {
         bool neg = false;
 #pragma unroll
-        for (int st = 0; st < MT; ++st) {
-          const int m = m0 + (st & ~(MG - 1)) + ((st & (MG - 1)) ^ pm);
-          if (l == max(m, an[s])) {  // E[l][col] (symmetries of d)
-            int col;
-            bool flip = false;
-            if (m >= an[s]) {
-              col = nv[s];
-            } else if (nv[s] > 0) {
-              col = m;
-              flip = ((m - nv[s]) & 1) != 0;
-            } else {
-              col = -m;
-            }
-            const RotXD e0 = p.start[(size_t)l * NN + L - 1 + col];
-            v[st][s] = flip ? -e0.m : e0.m;
-            kx[st][s] = e0.e;
-            vp[st][s] = 0.0;
-          }
-          neg |= kx[st][s] < 0;
-        }
-        scaled = __any_sync(0xffffffffu, neg) || scaled;
-      }
-      if constexpr (PL) {  // warp slots not started yet: their entries of the planes are 0
+        for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-          if (l >= wmin[s] || an[s] >= L) continue;
-#pragma unroll
-          for (int i = 0; i < MT; ++i) {
-            const int m = m0 + i;
-            if (m >= L) continue;
-            dl[((size_t)l * NN + L - 1 + m) * NN + L - 1 + nv[s]] = 0.0;
-            if (m > 0) dl[((size_t)l * NN + L - 1 - m) * NN + L - 1 - nv[s]] = 0.0;
-          }
-        }
+          for (int s = 0; s < S; ++s) neg |= kx[i][s] < 0;
+        scaled = __any_sync(0xffffffffu, neg);
       }
+    };
+    if (l >= wany) {  // some entry of the warp has started (warp-uniform)
+      if (scaled)
+        advance(std::true_type{});
+      else
+        advance(std::false_type{});
+    }
 
-      // the four weights of a lane's n in its sum-slot order:
-      // e^{-in gamma} flm[n] (order +m) and (-1)^n e^{in gamma} flm[-n] (order -m, times
-      // (-1)^m at the flush)
-      double Y[S][4];
-      if constexpr (contract) {
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-          const double2 g = eph[s], x = xa[s], y = xb[s];
-          const double sg = (nv[s] & 1) ? -1.0 : 1.0;
-          const double p0 = x.x * g.x - x.y * g.y, p1 = x.x * g.y + x.y * g.x;
-          const double q0 = sg * (y.x * g.x + y.y * g.y), q1 = sg * (y.y * g.x - y.x * g.y);
-          const double a0 = (cm & 2) ? q0 : p0, a1 = (cm & 2) ? q1 : p1;
-          const double b0 = (cm & 2) ? p0 : q0, b1 = (cm & 2) ? p1 : q1;
-          Y[s][0] = (cm & 1) ? a1 : a0;
-          Y[s][1] = (cm & 1) ? a0 : a1;
-          Y[s][2] = (cm & 1) ? b1 : b0;
-          Y[s][3] = (cm & 1) ? b0 : b1;
-        }
-      }
+    if (lc == kRotChunk - 1 || l == L - 1) {
+      __syncthreads();  // the next chunk's coefficients in place
+      ub ^= 1;
+      lc = 0;
+    } else {
+      ++lc;
+    }
+  }
+  cp_async_wait<0>();  // the pipeline's trailing (empty) copies
+}
 
-      // one degree of every started entry, branch-free so that the MT x S recurrences
-      // interleave; SC: with the 2^kx weights and the renormalisation
-      auto advance = [&](auto sc_tag) {
-        constexpr bool SC = decltype(sc_tag)::value;
+// ---------------------------------------------------------------------------------
+// rotation: the walk along n
+// ---------------------------------------------------------------------------------
+
+// a + b = hi + lo (|hi| >= |lo|), with a binary exponent: the running products of the tables
+struct DDX {
+  double h, l;
+  int e;
+};
+__device__ __forceinline__ DDX ddx_mul(DDX a, DDX b) {
+  const double p = a.h * b.h;
+  const double r = fma(a.h, b.h, -p) + fma(a.h, b.l, a.l * b.h);
+  const double h = p + r, l = r - (h - p);
+  int d;
+  DDX o;
+  o.h = frexp(h, &d);
+  if (o.h == 0.0) d = 0;
+  o.l = ldexp(l, -d);
+  o.e = a.e + b.e + d;
+  return o;
+}
+__device__ DDX ddx_pow(DDX b, int n) {  // b^n, n >= 0
+  DDX r{0.5, 0.0, 1};
+  while (n) {
+    if (n & 1) r = ddx_mul(r, b);
+    b = ddx_mul(b, b);
+    n >>= 1;
+  }
+  return r;
+}
+// the square root of a (a >= 0), as mantissa and exponent
+__device__ __forceinline__ RotXD ddx_sqrt(DDX a) {
+  if (a.e & 1) {
+    a.h *= 2.0;
+    a.l *= 2.0;
+    a.e -= 1;
+  }
+  RotXD r;
+  const double q = sqrt(a.h);
+  r.m = q > 0.0 ? q + (fma(-q, q, a.h) + a.l) / (2.0 * q) : 0.0;
+  r.e = a.e / 2;
+  r.pad = 0;
+  return r;
+}
+
+// W(j) = Gamma((j+1)/2) / (sqrt(pi) Gamma(j/2 + 1)): W(0) = 1, W(1) = 2/pi,
+// W(j) = W(j-2) (j-1)/j; from j = 32 the expansion of the logarithm of the gamma ratio in
+// 1/j (Bernoulli numbers), whose first omitted term is below 1e-17 there
+__device__ double rot_w(int j) {
+  if (j < 32) {
+    double w = (j & 1) ? 0.63661977236758134308 : 1.0;
+    for (int k = 2 + (j & 1); k <= j; k += 2) w = w * (double)(k - 1) / (double)k;
+    return w;
+  }
+  const double z = 0.5 * (double)j, i = 1.0 / z, i2 = i * i;
+  double s = 691.0 / 180224.0;
+  s = fma(s, i2, -31.0 / 18432.0);
+  s = fma(s, i2, 17.0 / 14336.0);
+  s = fma(s, i2, -1.0 / 640.0);
+  s = fma(s, i2, 1.0 / 192.0);
+  s = fma(s, i2, -1.0 / 8.0);
+  return exp(s * i) / sqrt(3.14159265358979323846 * z);
+}
+
+// Tables of one rotation (each of at most 2L entries): the phases, W, the powers of
+// cos(beta/2) and sin(beta/2), and (the last CTA) sqrt(k!), a scan of double-double products
+// so that the start values carry a few roundings only. With caller planes: the phases alone.
+constexpr int kRotTab = 1024;
+__global__ void __launch_bounds__(kRotTab) rotate_tables_kernel(RotParams p) {
+  const int L = p.L, NN = 2 * L - 1, tid = threadIdx.x;
+  if (!p.dl_in && blockIdx.x == gridDim.x - 1) {
+    __shared__ DDX tot[2][kRotTab];
+    const int per = (2 * L + kRotTab - 1) / kRotTab, k0 = tid * per;
+    DDX a{0.5, 0.0, 1};
+    auto times = [](DDX x, int k) {
+      int d;
+      DDX f{0.0, 0.0, 0};
+      f.h = frexp((double)(k > 0 ? k : 1), &d);
+      f.e = d;
+      return ddx_mul(x, f);
+    };
+    for (int k = k0; k < min(k0 + per, 2 * L); ++k) a = times(a, k);
+    int cur = 0;
+    tot[0][tid] = a;
+    __syncthreads();
+    for (int o = 1; o < kRotTab; o <<= 1) {
+      DDX t = tot[cur][tid];
+      if (tid >= o) t = ddx_mul(t, tot[cur][tid - o]);
+      tot[cur ^ 1][tid] = t;
+      cur ^= 1;
+      __syncthreads();
+    }
+    a = tid ? tot[cur][tid - 1] : DDX{0.5, 0.0, 1};
+    for (int k = k0; k < min(k0 + per, 2 * L); ++k) {
+      a = times(a, k);
+      p.sqf[k] = ddx_sqrt(a);
+    }
+    return;
+  }
+  const int i = blockIdx.x * kRotTab + tid;
+  if (i < NN) {
+    const double k = (double)(i - (L - 1));
+    double s, c;
+    sincos(-k * p.alpha, &s, &c);
+    p.ea[i] = make_double2(c, s);
+    sincos(-k * p.gamma, &s, &c);
+    p.eg[i] = make_double2(c, s);
+  }
+  if (!p.dl_in && i < 2 * L) {
+    p.w[i] = rot_w(i);
+    auto power = [i](double h, double l) {
+      int d;
+      DDX b;
+      b.h = frexp(h, &d);
+      b.l = ldexp(l, -d);
+      b.e = d;
+      const DDX r = ddx_pow(b, i);
+      RotXD o;
+      o.m = r.h + r.l;
+      o.e = r.e;
+      o.pad = 0;
+      return o;
+    };
+    p.cpow[i] = power(p.ch, p.cl);
+    p.spow[i] = power(p.sh, p.sl);
+  }
+}
+
+constexpr int kWalkThreads = 128;  // also the steps of a staged chunk
+constexpr int kWalkDead = -192;    // entries below 2^-192 do not contribute
+
+// The rotation. For fixed (l, m) the values along n obey
+//   a_n d_{m,n-1} + a_{n+1} d_{m,n+1} = 2 (n cos b - m)/sin b d_{m,n},
+//   a_n = sqrt((l+n)(l-n+1)),
+// and with d_{m,n} = g_n x_n, g_n^2 = W(l-n) W(l+n), the step is monic:
+//   x_{n-1} = -t x_n - x_{n+1},   t = A_n (m - n) + C_n,
+//   A_n = pi W(l-n) W(l+n) / sin b,   C_n = A_n n (1 - cos b).
+// A lane owns orders m of one degree l and walks n downwards, so the sum over n stays in its
+// registers and A, C and the weights g_n e^{-in gamma} flm[l, +-n] are warp-wide broadcasts:
+// two FP64 operations for a value and four for its products with flm[n] (order m) and, by
+// d_{-m,-n} = (-1)^{m-n} d_{m,n}, flm[-n] (order -m).
+// A walk is stable while the values grow or oscillate: it starts at n = l (closed form) and
+// ends at the centre n = m cos b of its oscillating range; the walk of order -m covers the
+// rest by the same symmetry. Half of the CTA's warps walk orders m >= 0, half the orders -m.
+// beta is folded to (0, pi/2] first (d(pi - b)_{m,n} = (-1)^{l+m} d(b)_{m,-n}), where m - n
+// and n (1 - cos b) keep t accurate.
+// Values below 2^-192 (the classically forbidden range) are carried as x 2^e and only
+// stepped; their products are left out: at most 2^-192 of a coefficient. The exponents are
+// renewed every G steps, between which a value grows by less than 2^100 (G = 4 for
+// sin(b/2) >= 2^-16, else 1). A non-finite coefficient makes its degree NaN, as a product
+// with a zero would.
+// Grid: (order tiles, degrees from the largest, maps). Bound by the FP64 pipe (six operations
+// per value) and the shared-memory broadcasts (48 bytes per step for the R orders of a lane),
+// with no reduction across lanes: L = 1024, one float64 map, 0.49-0.63 ms over beta (2.6-3.3 ms
+// with recurrences along the degree, whose sums over n crossed lanes, warps and a cluster).
+template <typename R2, int R, int G>
+__global__ void __launch_bounds__(kWalkThreads, 4) rotate_walk_kernel(RotParams p) {
+  // two staged chunks: (A, C) of each step, then its two weights; at the end the exchange
+  __shared__ __align__(16) double2 smem[2 * 3 * kWalkThreads];
+  double2* const sAC = smem;
+  double2* const sX = smem + 2 * kWalkThreads;
+  constexpr int kSpan = 32 * R;                          // orders of a warp
+  constexpr int kTile = kSpan * (kWalkThreads / 64);     // orders of a CTA
+  static_assert(sizeof(smem) >= (size_t)kTile * 4 * sizeof(double), "exchange");
+  const int L = p.L, NN = 2 * L - 1, l = L - 1 - (int)blockIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool neg = warp >= kWalkThreads / 64;            // this warp walks orders -m
+  const int mt = blockIdx.x * kTile;
+  const int mb = mt + (warp % (kWalkThreads / 64)) * kSpan + lane * R;
+  const size_t row = ((size_t)blockIdx.z * L + l) * NN + (L - 1);
+  if (mt > l) {  // orders beyond the degree: zeros
+    for (int i = tid; i < kTile; i += kWalkThreads)
+      if (mt + i < L) {
+        RotIO<R2>::put(p.out, row + mt + i, make_double2(0.0, 0.0));
+        RotIO<R2>::put(p.out, row - mt - i, make_double2(0.0, 0.0));
+      }
+    return;
+  }
+  // start values d_{M,l} = sqrt((2l)! / ((l+M)! (l-M)!)) cos^{l+M} sin^{l-M} of M = +-m
+  double v[R], vp[R];
+  int e[R];
+  int smin = l + 1, smax = -l - 1;  // least and largest last step over the warp
+  {
+    const RotXD f2 = p.sqf[2 * l];
+    const double ig = 1.0 / sqrt(p.w[0] * p.w[2 * l]);
 #pragma unroll
-        for (int g = 0; g < MT / MG; ++g) {
-          double x[V];
+    for (int r = 0; r < R; ++r) {
+      const int m = mb + r, M = neg ? -m : m;
+      v[r] = vp[r] = 0.0;
+      e[r] = 0;
+      if (m > l) continue;
+      const RotXD fa = p.sqf[l + M], fb = p.sqf[l - M], c = p.cpow[l + M], s = p.spow[l - M];
+      int d;
+      double x = frexp(f2.m / (fa.m * fb.m) * (c.m * s.m) * ig, &d);
+      const int ex = f2.e - fa.e - fb.e + c.e + s.e + d;
+      if (ex >= kWalkDead || x == 0.0)
+        x = ldexp(x, ex);
+      else
+        e[r] = ex;
+      v[r] = x;
+    }
+  }
+  int last[R];  // last n of each walk
 #pragma unroll
-          for (int u = 0; u < V; ++u) x[u] = 0.0;
+  for (int r = 0; r < R; ++r) {
+    const int c = (int)ceil((double)(mb + r) * p.cb);
+    last[r] = neg ? 1 - c : c;
+    if (mb + r <= l) {
+      smin = min(smin, last[r]);
+      smax = max(smax, last[r]);
+    }
+  }
+  smin = __reduce_min_sync(0xffffffffu, smin);
+  smax = __reduce_max_sync(0xffffffffu, smax);
+  // the CTA's least last step: that of its largest order's negative walk
+  const int mtop = min(l, mt + kTile - 1);
+  const int cmin = min((int)ceil((double)mt * p.cb), 1 - (int)ceil((double)mtop * p.cb));
+  const int nchunks = (l - cmin) / kWalkThreads + 1;
+
+  double q = (double)((neg ? -mb : mb) - l);  // M - n of the lane's first walk
+  double ap[R][2], an[R][2];  // products with flm[n] (order M) and flm[-n] (order -M)
 #pragma unroll
-          for (int is = 0; is < MG; ++is) {
-            const int st = g * MG + is;        // state slot
-            const int i = g * MG + (is ^ pm);  // order of the slot on this lane
-            const double4 uv = uvl[i];
+  for (int r = 0; r < R; ++r) ap[r][0] = ap[r][1] = an[r][0] = an[r][1] = 0.0;
+
+  // staging: thread tid holds step tid of a chunk
+  double2 xr, xl, ph;
+  double wa, wb;
+  auto fetch = [&](int ch) {
+    const int n = l - (ch * kWalkThreads + tid);
+    xr = xl = ph = make_double2(0.0, 0.0);
+    wa = wb = 0.0;
+    if (n >= -l) {
+      const int k = p.flip ? -n : n;  // the coefficient that stands for n
+      xr = RotIO<R2>::get(p.flm, row + k);
+      xl = RotIO<R2>::get(p.flm, row - k);
+      ph = p.eg[L - 1 + k];
+      wa = p.w[l - n];
+      wb = p.w[l + n];
+    }
+  };
+  bool bad = false;
+  auto stage = [&](int ch) {
+    const int n = l - (ch * kWalkThreads + tid), b = ch & 1;
+    const double ww = wa * wb, g = sqrt(ww), dn = (double)n;
+    const double A = fma(p.pis, ww, p.pisl * ww);
+    const double sp = (p.par & n & 1) ? -g : g;         // (-1)^n where sin, cos differ in sign
+    const double sn = ((p.par ^ 1) & n & 1) ? -g : g;   // times the (-1)^n of order -m
+    sAC[b * kWalkThreads + tid] = make_double2(A, A * fma(dn, p.y, dn * p.yl));
+    double2* const x = sX + 2 * (b * kWalkThreads + tid);
+    x[0] = make_double2(sp * (xr.x * ph.x - xr.y * ph.y),
+                                 sp * (xr.x * ph.y + xr.y * ph.x));
+    x[1] = make_double2(sn * (xl.x * ph.x + xl.y * ph.y),
+                                 sn * (xl.y * ph.x - xl.x * ph.y));
+    const double z = 0.0 * xr.x + 0.0 * xr.y + 0.0 * xl.x + 0.0 * xl.y;
+    bad |= z != z;
+  };
+  fetch(0);
+  stage(0);
+  int mode = 0;  // 0: nothing of the warp contributes yet, 1: some lanes do, 2: all do
+  if (__any_sync(0xffffffffu, mb <= l && e[0] == 0)) mode = 1;
 #pragma unroll
-            for (int s = 0; s < S; ++s) {
-              if (S > 1 && l < wmin[s]) continue;  // warp-uniform
-              double dv = v[st][s];
-              if constexpr (SC) dv *= pow2k(kx[st][s]);
-              if constexpr (contract) {
+  for (int r = 1; r < R; ++r)
+    if (__any_sync(0xffffffffu, mb + r <= l && e[r] == 0)) mode = 1;
+
+  auto renew = [&] {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) x[4 * is + c] = fma(dv, Y[s][c], x[4 * is + c]);
-              } else {
-                const int m = m0 + i;
-                if (an[s] < L && m < L) {
-                  dl[((size_t)l * NN + L - 1 + m) * NN + L - 1 + nv[s]] = dv;
-                  if (m > 0)
-                    dl[((size_t)l * NN + L - 1 - m) * NN + L - 1 - nv[s]] =
-                        ((m - nv[s]) & 1) ? -dv : dv;
-                }
-              }
-              if (step) {
-                const double t = fma(uv.z, nd[s], p.cb);
-                double vn = (uv.x * tn[s].x) * fma(t, v[st][s], -(uv.y * tn[s].y) * vp[st][s]);
-                double vc = v[st][s];
-                if constexpr (SC) {  // renormalise by up to 2^64 once |vn| >= 2^65
-                  const bool big =
-                      kx[st][s] < 0 && (__double2hiint(vn) & 0x7ff00000) > ((1023 + 64) << 20);
-                  const int sh = big ? min(64, -kx[st][s]) : 0;
-                  const double f = __hiloint2double((1023 - sh) << 20, 0);
-                  vn *= f;
-                  vc *= f;
-                  kx[st][s] += sh;
-                }
-                vp[st][s] = vc;
-                v[st][s] = vn;
-              }
-            }
-          }
-          if constexpr (contract) {
-            const double r = reduce_perm<V>(x);
-            if ((lane & (32 / V - 1)) == 0) sbuf[(lc * nw + warp) * (4 * MT) + g * V + mask] = r;
-          }
-        }
-        if constexpr (SC) {
-          bool neg = false;
+    for (int r = 0; r < R; ++r) {
+      if (e[r] < 0) {
+        const int x = ((__double2hiint(v[r]) >> 20) & 0x7ff) - 1022, en = e[r] + x;
+        const int sh = en >= kWalkDead ? e[r] : -x;
+        const double f = __hiloint2double((1023 + sh) << 20, 0);
+        v[r] *= f;
+        vp[r] *= f;
+        e[r] = en >= kWalkDead ? 0 : en;
+      }
+    }
+  };
+  for (int ch = 0; ch < nchunks; ++ch) {
+    __syncthreads();
+    const bool more = ch + 1 < nchunks;
+    if (more) fetch(ch + 1);
+    const int nt = l - ch * kWalkThreads;  // n of the chunk's first step
+    const double2* const ac = sAC + (ch & 1) * kWalkThreads;
+    const double2* const xx = sX + (ch & 1) * 2 * kWalkThreads;
+#pragma unroll 1
+    for (int k = 0; k < kWalkThreads && nt - k >= smin; k += G) {
+      // one value step of every walk
+      auto step = [&](int j) {
+        const double2 c = ac[k + j];
+        const double t0 = fma(q, c.x, c.y);
+        q += 1.0;
 #pragma unroll
-          for (int st = 0; st < MT; ++st)
-#pragma unroll
-            for (int s = 0; s < S; ++s) neg |= kx[st][s] < 0;
-          scaled = __any_sync(0xffffffffu, neg);
+        for (int r = 0; r < R; ++r) {
+          const double t = r == 0 ? t0 : fma(neg ? -(double)r : (double)r, c.x, t0);
+          const double x = fma(-t, v[r], -vp[r]);
+          vp[r] = v[r];
+          v[r] = x;
         }
       };
-      if (l >= wany) {  // some entry of the warp has started (warp-uniform)
-        if (scaled)
-          advance(std::true_type{});
-        else
-          advance(std::false_type{});
-      } else if constexpr (contract) {
+      if (mode == 2 && nt - k - (G - 1) >= smax) {
 #pragma unroll
-        for (int g = 0; g < MT / MG; ++g)
-          if ((lane & (32 / V - 1)) == 0) sbuf[(lc * nw + warp) * (4 * MT) + g * V + mask] = 0.0;
-      }
-
-      if (lc == kRotChunk - 1 || l == L - 1) {
-        __syncthreads();  // sums of the chunk and the next chunk's coefficients in place
-        if constexpr (contract) {
-          // this CTA's warps summed into cpart slot ck % 3
-          double* const cp = cpart + (ck % 3) * kRotChunk * 4 * MT;
-          const int nv4 = (lc + 1) * 4 * MT;
-          for (int e = tid; e < nv4; e += nt) {
-            const double* src = sbuf + (size_t)(e / (4 * MT)) * nw * 4 * MT + e % (4 * MT);
-            double t = 0.0;
+        for (int j = 0; j < G; ++j) {
+          const double2 xp = xx[2 * (k + j)], xn = xx[2 * (k + j) + 1];
 #pragma unroll
-            for (int w = 0; w < kRotThreads / 32; ++w)
-              if (w < nw) t += src[w * 4 * MT];
-            cp[e] = t;
+          for (int r = 0; r < R; ++r) {
+            ap[r][0] = fma(v[r], xp.x, ap[r][0]);
+            ap[r][1] = fma(v[r], xp.y, ap[r][1]);
+            an[r][0] = fma(v[r], xn.x, an[r][0]);
+            an[r][1] = fma(v[r], xn.y, an[r][1]);
           }
-          __syncthreads();  // sbuf free for the next chunk
-          if (ck > 0) {     // the previous chunk: every CTA has published it
-            cluster_wait();
-            rotate_flush<R2, MT>(p, cpart + ((ck - 1) % 3) * kRotChunk * 4 * MT, pb, plf, plc,
-                                 m0, rank);
-          }
-          cluster_arrive();
-          pb = b;
-          plf = l - lc;
-          plc = lc;
-          ++ck;
+          step(j);
         }
-        ub ^= 1;
-        lc = 0;
+      } else if (mode == 0) {
+#pragma unroll
+        for (int j = 0; j < G; ++j) step(j);
+        renew();
+        bool live = false;
+#pragma unroll
+        for (int r = 0; r < R; ++r) live |= e[r] == 0 && mb + r <= l;
+        if (__any_sync(0xffffffffu, live)) mode = 1;
       } else {
-        ++lc;
-      }
-    }
-    cp_async_wait<0>();  // the pipeline's trailing (empty) copies
-  }
-  if constexpr (contract) {
-    if (ck > 0) {
-      cluster_wait();
-      rotate_flush<R2, MT>(p, cpart + ((ck - 1) % 3) * kRotChunk * 4 * MT, pb, plf, plc, m0, rank);
-      cluster_arrive();  // no CTA leaves while others read its sums
-      cluster_wait();
-    }
-  }
-}
-
-// FP64 tensor-core step: D (8 x 8) += A (8 x 4) B (4 x 8), lane t holding A[t/4][t%4],
-// B[t%4][t/4] and D[t/4][2 (t%4) + {0, 1}] (mma.m8n8k4 .f64 fragments)
-__device__ __forceinline__ void dmma_884(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
-// The contraction on the FP64 tensor cores (one n per fetching lane, 8 orders per tile).
-// A warp owns a warp slot of 32 n (fetched as in rotate_lrec_kernel, one per lane) and the
-// tile's 8 orders; for the arithmetic lane t takes order m0 + t/4 and the 8 n of positions
-// 4j + t%4, j = 0..7, so its 8 recurrences are exactly its A fragments of 8 MMA steps. The
-// B fragments are the weights of those n: lane t supplies component t/4 (+m re, +m im,
-// -m re, -m im; zero for t/4 >= 4), read from a per-warp table that each lane fills for
-// its own n. D[order][component] is the warp's sum over its 32 n, so no shuffle reduction
-// runs; lanes with t%4 < 2 park their two components in the same per-warp slots as
-// rotate_lrec_kernel, and the cluster reduction is the same.
-// Dynamic shared memory: ring [D][3][nt] double2 | uvq [2][kRotChunk][8] double4 |
-// ybuf [nw][32][4] double | sbuf [kRotChunk][nw][32] | cpart [3][kRotChunk][32].
-template <typename R2>
-__global__ void __launch_bounds__(kRotThreads, 2) rotate_mma_kernel(RotParams p) {
-  extern __shared__ double4 smem4[];
-  constexpr int MT = 8, D = 4;
-  const int L = p.L, NN = 2 * L - 1;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nt = blockDim.x;
-  const int nw = p.nw, nr = p.nr, rank = blockIdx.x;
-  const int m0 = blockIdx.y * MT;
-  double2* const ring = reinterpret_cast<double2*>(smem4);
-  double4* const uvq = smem4 + (D * 3 * nt) / 2;
-  double* const ybuf = reinterpret_cast<double*>(uvq + 2 * kRotChunk * MT);
-  double* const sbuf = ybuf + nw * 32 * 4;
-  double* const cpart = sbuf + kRotChunk * nw * 4 * MT;
-  double* const yw = ybuf + warp * 32 * 4;
-
-  // the fetching lane's n (zigzag order, as rotate_lrec_kernel)
-  const int gw = warp * nr + rank;
-  const int wmin = 16 * gw;  // least |n| of the warp slot
-  const int jf = gw * 32 + lane;
-  const int nf = (jf & 1) ? -((jf + 1) >> 1) : (jf >> 1);
-  const bool okf = jf < NN;
-  const int nvf = okf ? nf : 0, anf = okf ? abs(nf) : L;
-  const double2 eph = okf ? p.eg[L - 1 + nf] : make_double2(0.0, 0.0);
-  // the arithmetic lane's order and n
-  const int row = lane >> 2, q = lane & 3;
-  const int m = m0 + row;
-  int nv[8], an[8];
-  double nd[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int jj = gw * 32 + 4 * j + q;
-    const int n = (jj & 1) ? -((jj + 1) >> 1) : (jj >> 1);
-    const bool ok = jj < NN;
-    nv[j] = ok ? n : 0;
-    an[j] = ok ? abs(n) : L;
-    nd[j] = (double)nv[j];
-  }
-  const int wlo = max(m0, wmin), whi = min(L - 1, max(m0 + MT - 1, wmin + 16));
-
-  int ck = 0, pb = 0, plf = 0, plc = 0;
-#pragma unroll 1
-  for (int b = 0; b < p.batch; ++b) {
-    {  // degrees below m0: the tile's rows are zero there
-      const int tot = m0 * 2 * MT;
-#pragma unroll 1
-      for (int e = rank * nt + tid; e < tot; e += nr * nt) {
-        const int l = e / (2 * MT), ci = e % (2 * MT), mm = m0 + (ci >> 1);
-        if (mm >= L || (mm == 0 && (ci & 1))) continue;
-        RotIO<R2>::put(p.out, ((size_t)b * L + l) * NN + L - 1 + ((ci & 1) ? -mm : mm),
-                       make_double2(0.0, 0.0));
-      }
-    }
-    const R2* const fb = reinterpret_cast<const R2*>(p.flm) + (size_t)b * L * NN + L - 1;
-    const unsigned rbase = (unsigned)__cvta_generic_to_shared(ring + tid);
-    const double2* tq = p.T + (size_t)m0 * L + min(anf, L - 1);
-    const R2* fq = fb + (size_t)m0 * NN + nvf;
-    int ll = m0;
-    auto issue = [&](int st) {  // the fetching lane's operands of degree ll into stage st
-      const bool vt = ll < L && ll >= wmin;
-      const unsigned r = rbase + (unsigned)(st * 3 * nt) * 16u;
-      cp_async<16>(r, tq, vt);
-      const bool vf = vt && anf <= ll;
-      cp_async<sizeof(R2)>(r + 16u * nt, fq, vf);
-      cp_async<sizeof(R2)>(r + 32u * nt, fq - 2 * nvf, vf);
-      if (ll + 1 < L) {
-        tq += L;
-        fq += NN;
-      }
-      ++ll;
-    };
-    rotate_stage<MT>(p, uvq, m0, m0);
-    cp_async_commit();
+        for (int j = 0; j < G; ++j) {
+          const double2 xp = xx[2 * (k + j)], xn = xx[2 * (k + j) + 1];
 #pragma unroll
-    for (int k = 0; k < D - 1; ++k) {
-      issue(k);
-      cp_async_commit();
-    }
-    cp_async_wait<D - 1>();
-    __syncthreads();
-
-    double v[8], vp[8];
-    int kx[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      v[j] = 0.0;
-      vp[j] = 0.0;
-      kx[j] = 0;
-    }
-    bool scaled = false;  // some lane of the warp carries a start value below 2^-960
-    int lc = 0, ub = 0, rs = 0;
-#pragma unroll 1
-    for (int l = m0; l < L; ++l) {
-      const bool step = l + 1 < L;
-      __syncwarp();  // every lane is done with the stage the next copies overwrite
-      issue(rs == 0 ? D - 1 : rs - 1);  // degree l + D - 1
-      if (lc == 0 && l + kRotChunk < L)
-        rotate_stage<MT>(p, uvq + (ub ^ 1) * kRotChunk * MT, l + kRotChunk, m0);
-      cp_async_commit();
-      cp_async_wait<D - 1>();
-      __syncwarp();  // the warp's copies of this degree are visible to all its lanes
-      const double2* const rg = ring + rs * 3 * nt + warp * 32;  // T of the warp's n
-      const int rso = rs;
-      rs = rs == D - 1 ? 0 : rs + 1;
-      double* const slot = sbuf + (lc * nw + warp) * (4 * MT);
-      if (l >= wmin) {  // some entry of the warp has started (warp-uniform)
-        {  // the weights of the fetching lane's n: e^{-in gamma} flm[n], (-1)^n e^{in gamma} flm[-n]
-          double2 xa, xb;
-          const double2* r = ring + rso * 3 * nt + tid;
-          if constexpr (sizeof(R2) == 16) {
-            xa = r[nt];
-            xb = r[2 * nt];
-          } else {
-            const float2 fa = *reinterpret_cast<const float2*>(r + nt);
-            const float2 fc = *reinterpret_cast<const float2*>(r + 2 * nt);
-            xa = make_double2(fa.x, fa.y);
-            xb = make_double2(fc.x, fc.y);
+          for (int r = 0; r < R; ++r) {
+            const double dv = e[r] == 0 && nt - k - j >= last[r] ? v[r] : 0.0;
+            ap[r][0] = fma(dv, xp.x, ap[r][0]);
+            ap[r][1] = fma(dv, xp.y, ap[r][1]);
+            an[r][0] = fma(dv, xn.x, an[r][0]);
+            an[r][1] = fma(dv, xn.y, an[r][1]);
           }
-          const double sg = (nvf & 1) ? -1.0 : 1.0;
-          double4 y;
-          y.x = xa.x * eph.x - xa.y * eph.y;
-          y.y = xa.x * eph.y + xa.y * eph.x;
-          y.z = sg * (xb.x * eph.x + xb.y * eph.y);
-          y.w = sg * (xb.y * eph.x - xb.x * eph.y);
-          reinterpret_cast<double4*>(yw)[lane] = y;
+          step(j);
         }
-        // entries starting at this degree (only inside the warp slot's start window)
-        if (l >= wlo && l <= whi) {
-          bool neg = false;
+        renew();
+        bool all = true;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            if (l == max(m, an[j])) {  // E[l][col] (symmetries of d)
-              int col;
-              bool flip = false;
-              if (m >= an[j]) {
-                col = nv[j];
-              } else if (nv[j] > 0) {
-                col = m;
-                flip = ((m - nv[j]) & 1) != 0;
-              } else {
-                col = -m;
-              }
-              const RotXD e0 = p.start[(size_t)l * NN + L - 1 + col];
-              v[j] = flip ? -e0.m : e0.m;
-              kx[j] = e0.e;
-              vp[j] = 0.0;
-            }
-            neg |= kx[j] < 0;
-          }
-          scaled = __any_sync(0xffffffffu, neg) || scaled;
-        }
-        __syncwarp();  // the weight table is written
-        const double4 uv = uvq[(ub * kRotChunk + lc) * MT + row];
-        auto advance = [&](auto sc_tag) {
-          constexpr bool SC = decltype(sc_tag)::value;
-          double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;  // two accumulators: even, odd j
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int k = 4 * j + q;
-            const double2 tk = rg[k];
-            const double y = row < 4 ? yw[k * 4 + row] : 0.0;
-            double dv = v[j];
-            if constexpr (SC) dv *= pow2k(kx[j]);
-            if (j & 1)
-              dmma_884(e0, e1, dv, y);
-            else
-              dmma_884(d0, d1, dv, y);
-            if (step) {
-              const double t = fma(uv.z, nd[j], p.cb);
-              double vn = (uv.x * tk.x) * fma(t, v[j], -(uv.y * tk.y) * vp[j]);
-              double vc = v[j];
-              if constexpr (SC) {  // renormalise by up to 2^64 once |vn| >= 2^65
-                const bool big =
-                    kx[j] < 0 && (__double2hiint(vn) & 0x7ff00000) > ((1023 + 64) << 20);
-                const int sh = big ? min(64, -kx[j]) : 0;
-                const double f = __hiloint2double((1023 - sh) << 20, 0);
-                vn *= f;
-                vc *= f;
-                kx[j] += sh;
-              }
-              vp[j] = vc;
-              v[j] = vn;
-            }
-          }
-          if (q < 2)
-            reinterpret_cast<double2*>(slot)[2 * row + q] = make_double2(d0 + e0, d1 + e1);
-          if constexpr (SC) {
-            bool neg = false;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) neg |= kx[j] < 0;
-            scaled = __any_sync(0xffffffffu, neg);
-          }
-        };
-        if (scaled)
-          advance(std::true_type{});
-        else
-          advance(std::false_type{});
-      } else if (q < 2) {
-        reinterpret_cast<double2*>(slot)[2 * row + q] = make_double2(0.0, 0.0);
-      }
-
-      if (lc == kRotChunk - 1 || l == L - 1) {
-        __syncthreads();  // sums of the chunk and the next chunk's coefficients in place
-        double* const cp = cpart + (ck % 3) * kRotChunk * 4 * MT;
-        const int nv4 = (lc + 1) * 4 * MT;
-        for (int e = tid; e < nv4; e += nt) {
-          const double* src = sbuf + (size_t)(e / (4 * MT)) * nw * 4 * MT + e % (4 * MT);
-          double t = 0.0;
-#pragma unroll
-          for (int w = 0; w < kRotThreads / 32; ++w)
-            if (w < nw) t += src[w * 4 * MT];
-          cp[e] = t;
-        }
-        __syncthreads();  // sbuf free for the next chunk
-        if (ck > 0) {     // the previous chunk: every CTA has published it
-          cluster_wait();
-          rotate_flush<R2, MT>(p, cpart + ((ck - 1) % 3) * kRotChunk * 4 * MT, pb, plf, plc, m0,
-                               rank);
-        }
-        cluster_arrive();
-        pb = b;
-        plf = l - lc;
-        plc = lc;
-        ++ck;
-        ub ^= 1;
-        lc = 0;
-      } else {
-        ++lc;
+        for (int r = 0; r < R; ++r) all &= e[r] == 0;
+        if (__all_sync(0xffffffffu, all)) mode = 2;
       }
     }
-    cp_async_wait<0>();
+    if (more) stage(ch + 1);
   }
-  if (ck > 0) {
-    cluster_wait();
-    rotate_flush<R2, MT>(p, cpart + ((ck - 1) % 3) * kRotChunk * 4 * MT, pb, plf, plc, m0, rank);
-    cluster_arrive();  // no CTA leaves while others read its sums
-    cluster_wait();
+  bad = __syncthreads_or(bad) || p.nan;
+
+  // the walks of -m hand their sums to those of m, which put both orders together
+  double* const ex = reinterpret_cast<double*>(smem);
+  const int o0 = mb - mt;
+  if (neg) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      ex[o0 + r] = ap[r][0];
+      ex[kTile + o0 + r] = ap[r][1];
+      ex[2 * kTile + o0 + r] = an[r][0];
+      ex[3 * kTile + o0 + r] = an[r][1];
+    }
+  }
+  __syncthreads();
+  if (!neg) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const double sg = ((mb + r) & 1) ? -1.0 : 1.0;
+      double* const x = ex + o0 + r;
+      const double br = x[0], bi = x[kTile], cr = x[2 * kTile], ci = x[3 * kTile];
+      x[0] = ap[r][0] + sg * cr;
+      x[kTile] = ap[r][1] + sg * ci;
+      x[2 * kTile] = br + sg * an[r][0];
+      x[3 * kTile] = bi + sg * an[r][1];
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < kTile && mt + i < L; i += kWalkThreads) {
+    const int m = mt + i;
+    const int odd = (p.par & m) ^ (p.flip & (l + m));
+    const double sg = bad ? CUDART_NAN : (odd & 1) ? -1.0 : 1.0;
+    const double2 a = p.ea[L - 1 + m];
+    double2 u = make_double2(0.0, 0.0), w = u;
+    if (m <= l) {
+      const double ur = sg * ex[i], ui = sg * ex[kTile + i];
+      const double wr = sg * ex[2 * kTile + i], wi = sg * ex[3 * kTile + i];
+      u = make_double2(ur * a.x - ui * a.y, ur * a.y + ui * a.x);
+      w = make_double2(wr * a.x + wi * a.y, wi * a.x - wr * a.y);
+    }
+    RotIO<R2>::put(p.out, row + m, u);
+    if (m > 0) RotIO<R2>::put(p.out, row - m, w);
   }
 }
 
@@ -970,9 +869,9 @@ struct RotShape {
   int mt, s, nw, nr;
 };
 
-// S n per lane so that a cluster of at most kRotMaxCluster CTAs of 8 warps covers all
-// 2L-1 n; MT (orders per cluster) as large as keeps two CTAs per SM busy, with MT x S
-// = 8 recurrences per lane at most (16 for L > 4096)
+// planes: S n per lane so that at most kRotMaxCluster CTAs of 8 warps cover all 2L-1 n; MT
+// (orders per tile) as large as keeps two CTAs per SM busy, with MT x S = 8 recurrences per
+// lane at most (16 for L > 4096)
 RotShape rotate_shape(int L, int sms) {
   const int NN = 2 * L - 1, slots = (NN + 31) / 32, wmax = kRotThreads / 32;
   RotShape r;
@@ -984,7 +883,7 @@ RotShape rotate_shape(int L, int sms) {
   if (r.s == 1) {
     r.mt = 8;
     while (r.mt > 2 && (long)r.nr * ((L + r.mt - 1) / r.mt) < 2L * sms) r.mt >>= 1;
-    // four orders per tile: CTAs of 4 warps in twice the clusters (L = 512: 0.60 -> 0.55 ms)
+    // four orders per tile: twice the CTAs, of 4 warps
     if (r.mt == 4 && r.nw == wmax && 2 * r.nr <= kRotMaxCluster) {
       r.nw /= 2;
       r.nr *= 2;
@@ -995,82 +894,19 @@ RotShape rotate_shape(int L, int sms) {
   return r;
 }
 
-template <typename R2, int MT, int S, bool PL>
+template <int MT, int S>
 cudaError_t launch_lrec(const RotParams& p, cudaStream_t s) {
-  // ring, uvq, and with the contraction sbuf and cpart (rotate_lrec_kernel)
-  const size_t nt = 32 * (size_t)p.nw;
-  const size_t smem = (size_t)rot_depth<S>() * S * 3 * nt * 16 + 2 * kRotChunk * MT * 32 +
-                      (!PL ? ((size_t)kRotChunk * p.nw * 4 * MT + 3 * kRotChunk * 4 * MT) * 8 : 0);
-  void (*kern)(RotParams) = rotate_lrec_kernel<R2, MT, S, PL>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  const size_t nt = 32 * (size_t)p.nw;  // ring and uvq (rotate_lrec_kernel)
+  const size_t smem = (size_t)rot_depth<S>() * S * nt * 16 + 2 * kRotChunk * MT * 32;
+  void (*kern)(RotParams) = rotate_lrec_kernel<MT, S>;
+  const cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)p.nr, (unsigned)((p.L + MT - 1) / MT), 1);
-  cfg.blockDim = dim3((unsigned)(32 * p.nw), 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)p.nr;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, p);
+  kern<<<dim3((unsigned)p.nr, (unsigned)((p.L + MT - 1) / MT)), (unsigned)nt, smem, s>>>(p);
+  return cudaGetLastError();
 }
 
-template <typename R2>
-cudaError_t launch_mma(const RotParams& p, cudaStream_t s) {
-  constexpr int MT = 8;
-  // ring, uvq, ybuf, sbuf and cpart (rotate_mma_kernel)
-  const size_t nt = 32 * (size_t)p.nw;
-  const size_t smem = (size_t)4 * 3 * nt * 16 + 2 * kRotChunk * MT * 32 +
-                      ((size_t)p.nw * 32 * 4 + (size_t)kRotChunk * p.nw * 4 * MT +
-                       3 * kRotChunk * 4 * MT) * 8;
-  void (*kern)(RotParams) = rotate_mma_kernel<R2>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)p.nr, (unsigned)((p.L + MT - 1) / MT), 1);
-  cfg.blockDim = dim3((unsigned)(32 * p.nw), 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)p.nr;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (p.nr > kRotMaxCluster) {  // non-portable cluster size: launch only where one fits
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    int nclusters = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg);
-    if (e != cudaSuccess || nclusters < 1) {
-      (void)cudaGetLastError();
-      return cudaErrorNotSupported;
-    }
-  }
-  return cudaLaunchKernelEx(&cfg, kern, p);
-}
-
-template <typename R2, bool PL>
-cudaError_t launch_shape(const RotParams& p, const RotShape& sh, cudaStream_t s) {
-  switch (sh.s * 16 + sh.mt) {
-    case 16 + 8: return launch_lrec<R2, 8, 1, PL>(p, s);
-    case 16 + 4: return launch_lrec<R2, 4, 1, PL>(p, s);
-    case 16 + 2: return launch_lrec<R2, 2, 1, PL>(p, s);
-    case 32 + 4: return launch_lrec<R2, 4, 2, PL>(p, s);
-    case 64 + 2: return launch_lrec<R2, 2, 4, PL>(p, s);
-    case 128 + 2: return launch_lrec<R2, 2, 8, PL>(p, s);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-template <typename R2>
-cudaError_t rotate_launch(RotParams p, cudaStream_t s) {
+cudaError_t planes_launch(RotParams p, cudaStream_t s) {
   const int L = p.L, NN = 2 * L - 1;
   const double c = std::cos(0.5 * p.beta), sn = std::sin(0.5 * p.beta);
   p.cb = std::cos(p.beta);
@@ -1079,18 +915,8 @@ cudaError_t rotate_launch(RotParams p, cudaStream_t s) {
   p.cs2 = (c * sn) * (c * sn);
   p.c_neg = c < 0.0;
   p.s_neg = sn < 0.0;
-  rotate_phase_kernel<<<(NN + 255) / 256, 256, 0, s>>>(p);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if (p.dl_in) {
-    const long warps = (long)p.batch * L * NN;
-    long blocks = (warps + 7) / 8;
-    if (blocks > 65535L * 16) blocks = 65535L * 16;
-    rotate_planes_kernel<R2><<<(unsigned)blocks, 256, 0, s>>>(p);
-    return cudaGetLastError();
-  }
   int dev = 0, sms = 0;
-  e = cudaGetDevice(&dev);
+  cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   const RotShape sh = rotate_shape(L, sms);
@@ -1104,20 +930,73 @@ cudaError_t rotate_launch(RotParams p, cudaStream_t s) {
   rotate_start_final_kernel<<<dim3(nb, L), 128, 0, s>>>(p);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (p.flm) {
-    const int slots = (NN + 31) / 32, wmax = kRotThreads / 32;
-    if (sh.s == 2 && slots <= 2 * kRotMaxCluster * wmax) {
-      // up to 4096 n (L <= 2048): the tensor-core kernel with one n per lane in clusters of
-      // up to 16 CTAs, where the device has them; else two n per lane below
-      RotParams q = p;
-      q.nw = wmax;
-      q.nr = (slots + wmax - 1) / wmax;
-      e = launch_mma<R2>(q, s);
-      if (e != cudaErrorNotSupported) return e;
-    }
-    if (sh.s == 1 && sh.mt == 8) return launch_mma<R2>(p, s);
+  switch (sh.s * 16 + sh.mt) {
+    case 16 + 8: return launch_lrec<8, 1>(p, s);
+    case 16 + 4: return launch_lrec<4, 1>(p, s);
+    case 16 + 2: return launch_lrec<2, 1>(p, s);
+    case 32 + 4: return launch_lrec<4, 2>(p, s);
+    case 64 + 2: return launch_lrec<2, 4>(p, s);
+    case 128 + 2: return launch_lrec<2, 8>(p, s);
+    default: return cudaErrorInvalidValue;
   }
-  return p.flm ? launch_shape<R2, false>(p, sh, s) : launch_shape<double2, true>(p, sh, s);
+}
+
+template <typename R2, int R, int G>
+cudaError_t launch_walk(const RotParams& p, cudaStream_t s) {
+  constexpr int tile = 16 * R * (kWalkThreads / 32);
+  const long grid_z = 65535;  // maps per launch
+  for (long b = 0; b < p.batch; b += grid_z) {
+    RotParams q = p;
+    const size_t off = (size_t)b * p.L * (2 * (size_t)p.L - 1);
+    q.flm = static_cast<const R2*>(p.flm) + off;
+    q.out = static_cast<R2*>(p.out) + off;
+    const unsigned nz = (unsigned)(p.batch - b < grid_z ? p.batch - b : grid_z);
+    rotate_walk_kernel<R2, R, G>
+        <<<dim3((unsigned)((p.L + tile - 1) / tile), (unsigned)p.L, nz), kWalkThreads, 0, s>>>(q);
+  }
+  return cudaGetLastError();
+}
+
+template <typename R2>
+cudaError_t rotate_launch(RotParams p, cudaStream_t s) {
+  const int L = p.L, NN = 2 * L - 1;
+  // beta folded to b in (0, pi/2]: cos and sin of b/2 in double-double
+  long double c = cosl(0.5L * p.beta), sn = sinl(0.5L * p.beta);
+  p.nan = !std::isfinite(p.beta);
+  if (p.nan) c = sn = 0.70710678118654752440L;
+  p.par = (c < 0.0L) != (sn < 0.0L);
+  c = fabsl(c);
+  sn = fabsl(sn);
+  p.flip = c < sn;
+  if (p.flip) std::swap(c, sn);
+  sn = fmaxl(sn, ldexpl(1.0L, -101));  // below, the rotation is the identity to rounding
+  p.ch = (double)c;
+  p.cl = (double)(c - p.ch);
+  p.sh = (double)sn;
+  p.sl = (double)(sn - p.sh);
+  p.cb = (double)((c - sn) * (c + sn));
+  // hi + lo: a rounding of these would be the same in every step and add up along the walk
+  const long double y = 2.0L * sn * sn, pis = 3.14159265358979323846264338L / (2.0L * sn * c);
+  p.y = (double)y;
+  p.yl = (double)(y - p.y);
+  p.pis = (double)pis;
+  p.pisl = (double)(pis - p.pis);
+  const int n = p.dl_in ? NN : 2 * L;
+  rotate_tables_kernel<<<(n + kRotTab - 1) / kRotTab + (p.dl_in ? 0 : 1), kRotTab, 0, s>>>(p);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  if (p.dl_in) {
+    const long warps = (long)p.batch * L * NN;
+    long blocks = (warps + 7) / 8;
+    if (blocks > 65535L * 16) blocks = 65535L * 16;
+    rotate_planes_kernel<R2><<<(unsigned)blocks, 256, 0, s>>>(p);
+    return cudaGetLastError();
+  }
+  if (sn < 0x1p-16L) return launch_walk<R2, 2, 1>(p, s);
+  // two orders per lane leave enough warps up to here (L = 1024, beta = 0.2 / 1.5: 626 / 485 us
+  // against 664 / 473 with four; L = 1500: 1784 / 1412 against 1803 / 1340), four need fewer
+  // broadcasts per order beyond (L = 2048: 4155 / 3222 us against 4282 / 3463)
+  return L < 1600 ? launch_walk<R2, 2, 4>(p, s) : launch_walk<R2, 4, 4>(p, s);
 }
 
 }  // namespace
@@ -1125,29 +1004,34 @@ cudaError_t rotate_launch(RotParams p, cudaStream_t s) {
 static size_t rot_align(size_t b) { return (b + 255) & ~(size_t)255; }
 
 size_t rotate_workspace_bytes(int L) {
-  const size_t NN = 2 * (size_t)L - 1, G = ((size_t)L + kRotSeg - 1) / kRotSeg;
-  return rot_align((size_t)L * L * sizeof(double2)) + rot_align((size_t)L * L * sizeof(double4)) +
-         rot_align((size_t)L * NN * sizeof(RotXD)) + rot_align(G * NN * sizeof(RotXD)) +
-         2 * rot_align(NN * sizeof(double2));
+  RotParams p{};
+  p.L = L;
+  return rotate_bind_workspace(p, nullptr);
 }
 
-void rotate_bind_workspace(RotParams& p, void* ws) {
-  char* c = static_cast<char*>(ws);
+size_t rotate_bind_workspace(RotParams& p, void* ws) {
   const size_t L = (size_t)p.L, NN = 2 * L - 1, G = (L + kRotSeg - 1) / kRotSeg;
-  p.T = reinterpret_cast<double2*>(c);
-  c += rot_align(L * L * sizeof(double2));
-  p.UVQ = reinterpret_cast<double4*>(c);
-  c += rot_align(L * L * sizeof(double4));
-  p.start = reinterpret_cast<RotXD*>(c);
-  c += rot_align(L * NN * sizeof(RotXD));
-  p.carry = reinterpret_cast<RotXD*>(c);
-  c += rot_align(G * NN * sizeof(RotXD));
-  p.ea = reinterpret_cast<double2*>(c);
-  c += rot_align(NN * sizeof(double2));
-  p.eg = reinterpret_cast<double2*>(c);
+  char* const base = static_cast<char*>(ws);
+  size_t off = 0;
+  auto carve = [&](auto*& x, size_t n) {
+    x = reinterpret_cast<std::remove_reference_t<decltype(x)>>(base + off);
+    off += rot_align(n * sizeof(*x));
+  };
+  carve(p.ea, NN);
+  carve(p.eg, NN);
+  carve(p.w, 2 * L);
+  carve(p.sqf, 2 * L);
+  carve(p.cpow, 2 * L);
+  carve(p.spow, 2 * L);
+  carve(p.T, L * L);
+  carve(p.UVQ, L * L);
+  carve(p.start, L * NN);
+  carve(p.carry, G * NN);
+  return off;
 }
 
-cudaError_t launch_rotate(bool fp64, RotParams p, cudaStream_t s) {
+cudaError_t launch_rotate(bool fp64, const RotParams& p, cudaStream_t s) {
+  if (!p.flm) return planes_launch(p, s);
   return fp64 ? rotate_launch<double2>(p, s) : rotate_launch<float2>(p, s);
 }
 
