@@ -277,7 +277,7 @@ int s2b_batch_set_option(s2b_batch* batch, int key, int value);
  * replaces s2fft.utils.rotation.rotate_flms (s2fft/utils/rotation.py:9-64). flm and out
  * are [batch][L][2L-1] complex (double for precision S2B_F64, float for S2B_F32); the
  * arithmetic is double in both. dl == NULL: the Wigner-d values at beta are generated
- * on the device by the three-term recurrence in the degree of every (m, n) (upstream
+ * on the device by the three-term recurrence along n of every (l, m) (upstream
  * builds the planes with Risbo's recursion, s2fft/recursions/risbo.py:4-120; the two
  * agree to rounding), L <= 8192; otherwise dl holds them in the layout of upstream's
  * generate_rotate_dls, [L][2L-1][2L-1] float64 with d^l_{m,n} at [l][L-1+m][L-1+n].

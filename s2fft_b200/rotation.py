@@ -7,7 +7,7 @@
     flm'[l, m] = exp(-i m alpha) sum_n d^l_{m,n}(beta) exp(-i n gamma) flm[l, n].
 
 Without ``dl_array`` the Wigner-d values at beta are generated on the device by the
-three-term recurrence in the degree of every (m, n), fused with the contraction (upstream
+three-term recurrence along n of every (l, m), fused with the contraction (upstream
 builds the planes with Risbo's recursion, s2fft/recursions/risbo.py:4-120; the two agree
 to rounding); with it (the layout of ``generate_rotate_dls``, rotation.py:75-96) only the
 contraction runs. The arithmetic is double; complex64 inputs are returned as
