@@ -561,8 +561,7 @@ template <typename Real, bool DUAL, int T, int W, int R, int SYM>
 static cudaError_t launch_fwd2_cfg(const Fwd2Params& p, cudaStream_t s) {
   using Lay = Fwd2Layout<Real, DUAL, T, W, R, SYM>;
   auto kern = lat_fwd2_kernel<Real, DUAL, T, W, R, SYM>;
-  cudaError_t err =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::total);
+  cudaError_t err = func_limits(kern, Lay::total);
   if (err != cudaSuccess) return err;
   const int ntiles = (p.nrings + Lay::NRT - 1) / Lay::NRT;
   dim3 grid(ntiles, (p.NB / 2) * (p.Mst1 ? p.nseg : 1), p.nhalf * p.batch);
@@ -615,8 +614,7 @@ static cudaError_t launch_fwd2_batch_cfg(const Fwd2Params* ps, int n, int* count
                                          cudaStream_t s) {
   using Lay = Fwd2Layout<Real, DUAL, T, 4, R, SYM>;
   auto kern = lat_fwd2_persistent<Real, DUAL, T, 4, R, SYM>;
-  cudaError_t err =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::total);
+  cudaError_t err = func_limits(kern, Lay::total);
   if (err != cudaSuccess) return err;
   Fwd2Batch w{};
   w.nplans = n;

@@ -143,6 +143,16 @@ __device__ __forceinline__ void chain_enter() {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
+cudaError_t func_limits_of(const void* kernel, int smem, int carveout);  // stages.cu
+
+// Dynamic shared memory limit (at least smem bytes) and, unless carveout < 0, shared-memory
+// carveout of a kernel on the current device: set when they change instead of before every
+// launch. The limit is only raised, so that a launch from another thread keeps its own.
+template <typename... KArgs>
+inline cudaError_t func_limits(void (*kernel)(KArgs...), size_t smem, int carveout = -1) {
+  return func_limits_of(reinterpret_cast<const void*>(kernel), (int)smem, carveout);
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                   cudaStream_t s, Args&&... args) {

@@ -8,7 +8,10 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <map>
+#include <mutex>
 #include <type_traits>
+#include <utility>
 
 #include "s2b_dev.h"
 #include "s2b_internal.h"
@@ -514,6 +517,31 @@ cudaError_t launch_sub(bool fp64, long n, const void* x, const void* y, void* z,
   else
     sub_kernel<float><<<grid_for(n), 256, 0, s>>>(n, (const float*)x, (const float*)y, (float*)z);
   return cudaGetLastError();
+}
+
+// What the current process has set, per kernel and device (one entry per kernel instance).
+cudaError_t func_limits_of(const void* kernel, int smem, int carveout) {
+  struct Limits {
+    int smem = 0, carveout = -1;
+  };
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, Limits> set;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  Limits& l = set[{kernel, dev}];
+  if (smem > l.smem) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    l.smem = smem;
+  }
+  if (carveout >= 0 && carveout != l.carveout) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
+    if (e != cudaSuccess) return e;
+    l.carveout = carveout;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace s2b
