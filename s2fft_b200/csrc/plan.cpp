@@ -2370,10 +2370,18 @@ static int build_wigner(s2b_plan* p) {
   return S2B_OK;
 }
 
-// fban | per stream: (tmp | sub-transform workspace)
-static size_t wigner_slot(const s2b_plan* p) { return align256(p->ws_w_tmp) + align256(p->ws_w_sub); }
+static void drop_aux(s2b_plan* p) {
+  if (p->aux) cudaStreamDestroy(p->aux);
+  if (p->aux_fork) cudaEventDestroy(p->aux_fork);
+  if (p->aux_join) cudaEventDestroy(p->aux_join);
+  p->aux = nullptr;
+  p->aux_fork = p->aux_join = nullptr;
+}
+
+// fban | per slice: coefficients | per stream: sub-transform workspace
 static size_t wigner_ws(const s2b_plan* p) {
-  return align256(p->ws_w_fban) + (size_t)std::max(1, p->nwstream) * wigner_slot(p);
+  return align256(p->ws_w_fban) + p->subs.size() * align256(p->ws_w_tmp) +
+         (size_t)std::max(1, p->nwstream) * align256(p->ws_w_sub);
 }
 
 static int run_wigner(s2b_plan* p, bool forward, const void* in, void* out, char* ws,
@@ -2384,29 +2392,27 @@ static int run_wigner(s2b_plan* p, bool forward, const void* in, void* out, char
   char* fban = ws;
   const size_t slice = (size_t)d.batch * p->npix * 2 * p->rsz;
   int rc;
-  if (forward) S2B_CK(launch_gamma_forward(p->fp64, in, fban, d.batch, d.N, p->npix, d.reality, s));
+  if (forward)
+    S2B_CK(launch_gamma_forward(p->fp64, in, fban, d.batch, d.N, p->npix, d.reality, s));
+  else
+    S2B_CK(launch_gather_slices(p->fp64, in, tmp, tstride, d.batch, d.N, d.L, n0, nsub, d.reality, s));
   if (K > 1) {
     std::lock_guard<std::mutex> lk(p->fork_mu);
     S2B_CK(cudaEventRecord(p->wfork, s));
+    // the slices run side by side already: their low orders follow in the same stream instead
+    // of on a stream of their own (four event calls per slice and direction)
+    drop_aux(sub);
     for (int k = 0; k < K; ++k) S2B_CK(cudaStreamWaitEvent(p->wstream[k], p->wfork, 0));
   }
   rc = S2B_OK;
   for (int n = n0; n < d.N && !rc; ++n) {
     const int k = (n - n0) % K;
     cudaStream_t sk = K > 1 ? p->wstream[k] : s;
-    char* tmp = fban + align256(p->ws_w_fban) + (size_t)k * wigner_slot(p);
-    char* subws = tmp + align256(p->ws_w_tmp);
-    s2b_plan* sub = p->subs[n - n0];
+    char* subws = sub_ws + (size_t)k * align256(p->ws_w_sub);
+    char* coef = tmp + (size_t)(n - n0) * align256(p->ws_w_tmp);
     char* band = fban + (size_t)(d.N - 1 + n) * slice;
-    cudaError_t e = cudaSuccess;
-    if (!forward) {
-      e = launch_gather_n(p->fp64, in, tmp, d.batch, d.N, d.L, n, d.reality && n == 0, sk);
-      if (e == cudaSuccess) rc = exec_call(sub, 0, tmp, band, subws, sk);
-    } else {
-      rc = exec_call(sub, 1, band, tmp, subws, sk);
-      if (!rc) e = launch_scatter_n(p->fp64, tmp, out, d.batch, d.N, d.L, n, d.L_lower, sk);
-    }
-    if (e != cudaSuccess) rc = fail(S2B_ERR_CUDA, std::string("Wigner gather/scatter: ") + cudaGetErrorString(e));
+    s2b_plan* sub = p->subs[n - n0];
+    rc = forward ? exec_call(sub, 1, band, coef, subws, sk) : exec_call(sub, 0, coef, band, subws, sk);
   }
   if (K > 1) {
     // join every forked stream back to the caller's stream, after an error too, so that no
@@ -2418,11 +2424,16 @@ static int run_wigner(s2b_plan* p, bool forward, const void* in, void* out, char
       if (e != cudaSuccess && !rc) rc = fail(S2B_ERR_CUDA, std::string("Wigner join: ") + cudaGetErrorString(e));
     }
   }
+  const int nsub = (int)p->subs.size();
   if (rc) return rc;
+  char* tmp = fban + align256(p->ws_w_fban);
+  char* sub_ws = tmp + nsub * align256(p->ws_w_tmp);
   if (!forward) {
+  const long tstride = (long)(align256(p->ws_w_tmp) / (2 * p->rsz));
     S2B_CK(launch_gamma_inverse(p->fp64, fban, out, d.batch, d.N, p->npix, d.reality, s));
-  } else if (d.reality) {
-    S2B_CK(launch_wigner_mirror(p->fp64, out, d.batch, d.N, d.L, s));
+  } else {
+    S2B_CK(launch_scatter_slices(p->fp64, tmp, tstride, out, d.batch, d.N, d.L, n0, nsub, d.L_lower, s));
+    if (d.reality) S2B_CK(launch_wigner_mirror(p->fp64, out, d.batch, d.N, d.L, s));
   }
   return S2B_OK;
 }
@@ -2528,9 +2539,7 @@ int s2b_plan_destroy(s2b_plan* p) {
   if (!p) return S2B_OK;
   for (s2b_plan* sp : p->subs) s2b_plan_destroy(sp);
   for (void* a : p->allocs) cudaFree(a);
-  if (p->aux) cudaStreamDestroy(p->aux);
-  if (p->aux_fork) cudaEventDestroy(p->aux_fork);
-  if (p->aux_join) cudaEventDestroy(p->aux_join);
+  drop_aux(p);
   for (int k = 0; k < s2b_plan::kMaxWStreams; ++k) {
     if (p->wstream[k]) cudaStreamDestroy(p->wstream[k]);
     if (p->wjoin[k]) cudaEventDestroy(p->wjoin[k]);

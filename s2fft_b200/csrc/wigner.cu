@@ -28,42 +28,49 @@ static int wgrid(long n) {
 // (wigner.py:176-187, spherical.py:176-208); the complex transform that follows does the
 // same when the orders are weighted by 0 (m < 0), 1 (m = 0) and 2 (m > 0) and the gamma DFT
 // keeps the real part of the slice.
+// The slices n = n0 .. n0 + K - 1 of every map, slice k to tmp + k stride. One launch for all of
+// them (one per slice made a fifth of the launches of an L = 128, N = 8 call).
 template <typename Real>
-__global__ void gather_n_kernel(const W2<Real>* flmn, W2<Real>* tmp, int B, int N, int L, int n,
-                                int real0) {
-  const long per = (long)L * (2 * L - 1);
-  const long total = per * B;
+__global__ void gather_slices_kernel(const W2<Real>* flmn, W2<Real>* tmp, long stride, int B, int N,
+                                     int L, int n0, int K, int real0) {
+  const int M = 2 * L - 1, per = L * M;
   const double pi = 3.141592653589793;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
-       i += (long)gridDim.x * blockDim.x) {
-    const long b = i / per, r = i % per;
-    const int l = (int)(r / (2 * L - 1));
-    const int m = (int)(r % (2 * L - 1)) - (L - 1);
-    double f = ((n & 1) ? -1.0 : 1.0) * sqrt((2.0 * l + 1.0) / (16.0 * pi * pi * pi));
-    if (real0) f *= m < 0 ? 0.0 : (m == 0 ? 1.0 : 2.0);
-    W2<Real> v = flmn[(b * (2 * N - 1) + (N - 1 + n)) * per + r];
-    v.x = (Real)(v.x * f);
-    v.y = (Real)(v.y * f);
-    tmp[i] = v;
+  for (long z = blockIdx.y; z < (long)B * K; z += gridDim.y) {
+    const int k = (int)(z % K), n = n0 + k;
+    const long b = z / K;
+    const W2<Real>* const src = flmn + (b * (2 * N - 1) + (N - 1 + n)) * per;
+    W2<Real>* const dst = tmp + k * stride + b * per;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < per; r += gridDim.x * blockDim.x) {
+      const int l = r / M, m = r % M - (L - 1);
+      double f = ((n & 1) ? -1.0 : 1.0) * sqrt((2.0 * l + 1.0) / (16.0 * pi * pi * pi));
+      if (real0 && n == 0) f *= m < 0 ? 0.0 : (m == 0 ? 1.0 : 2.0);
+      W2<Real> v = src[r];
+      v.x = (Real)(v.x * f);
+      v.y = (Real)(v.y * f);
+      dst[r] = v;
+    }
   }
 }
 
-// flmn[b][N-1+n][l][c] = (-1)^n sqrt(4pi/(2l+1)) tmp[b][l][c]  (l >= L0; else 0)
+// flmn[b][N-1+n][l][c] = (-1)^n sqrt(4pi/(2l+1)) tmp[k][b][l][c]  (l >= L0; else 0), n = n0 + k
 template <typename Real>
-__global__ void scatter_n_kernel(const W2<Real>* tmp, W2<Real>* flmn, int B, int N, int L, int n,
-                                 int L0) {
-  const long per = (long)L * (2 * L - 1);
-  const long total = per * B;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
-       i += (long)gridDim.x * blockDim.x) {
-    const long b = i / per, r = i % per;
-    const int l = (int)(r / (2 * L - 1));
-    W2<Real> v = tmp[i];
-    double f = 0.0;
-    if (l >= L0) f = ((n & 1) ? -1.0 : 1.0) * sqrt(4.0 * 3.141592653589793 / (2.0 * l + 1.0));
-    v.x = (Real)(v.x * f);
-    v.y = (Real)(v.y * f);
-    flmn[(b * (2 * N - 1) + (N - 1 + n)) * per + r] = v;
+__global__ void scatter_slices_kernel(const W2<Real>* tmp, long stride, W2<Real>* flmn, int B, int N,
+                                      int L, int n0, int K, int L0) {
+  const int M = 2 * L - 1, per = L * M;
+  for (long z = blockIdx.y; z < (long)B * K; z += gridDim.y) {
+    const int k = (int)(z % K), n = n0 + k;
+    const long b = z / K;
+    const W2<Real>* const src = tmp + k * stride + b * per;
+    W2<Real>* const dst = flmn + (b * (2 * N - 1) + (N - 1 + n)) * per;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < per; r += gridDim.x * blockDim.x) {
+      const int l = r / M;
+      W2<Real> v = src[r];
+      double f = 0.0;
+      if (l >= L0) f = ((n & 1) ? -1.0 : 1.0) * sqrt(4.0 * 3.141592653589793 / (2.0 * l + 1.0));
+      v.x = (Real)(v.x * f);
+      v.y = (Real)(v.y * f);
+      dst[r] = v;
+    }
   }
 }
 
@@ -175,25 +182,32 @@ __global__ void gamma_forward_kernel(const void* f, W2<Real>* fban, int B, int N
   }
 }
 
-cudaError_t launch_gather_n(bool fp64, const void* flmn, void* tmp, int B, int N, int L, int n,
-                            int real0, cudaStream_t s) {
-  const long tot = (long)B * L * (2 * L - 1);
+static dim3 slices_grid(int B, int L, int K) {
+  const long x = ((long)L * (2 * L - 1) + 255) / 256, y = (long)B * K;
+  return dim3((unsigned)(x < 4096 ? x : 4096), (unsigned)(y < 65535 ? y : 65535));
+}
+
+cudaError_t launch_gather_slices(bool fp64, const void* flmn, void* tmp, long stride, int B, int N,
+                                 int L, int n0, int K, int real0, cudaStream_t s) {
+  const dim3 g = slices_grid(B, L, K);
   if (fp64)
-    gather_n_kernel<double><<<wgrid(tot), 256, 0, s>>>((const double2*)flmn, (double2*)tmp, B, N, L, n,
-                                                       real0);
+    gather_slices_kernel<double><<<g, 256, 0, s>>>((const double2*)flmn, (double2*)tmp, stride, B, N,
+                                                   L, n0, K, real0);
   else
-    gather_n_kernel<float><<<wgrid(tot), 256, 0, s>>>((const float2*)flmn, (float2*)tmp, B, N, L, n,
-                                                      real0);
+    gather_slices_kernel<float><<<g, 256, 0, s>>>((const float2*)flmn, (float2*)tmp, stride, B, N, L,
+                                                  n0, K, real0);
   return cudaGetLastError();
 }
 
-cudaError_t launch_scatter_n(bool fp64, const void* tmp, void* flmn, int B, int N, int L, int n,
-                             int L0, cudaStream_t s) {
-  const long tot = (long)B * L * (2 * L - 1);
+cudaError_t launch_scatter_slices(bool fp64, const void* tmp, long stride, void* flmn, int B, int N,
+                                  int L, int n0, int K, int L0, cudaStream_t s) {
+  const dim3 g = slices_grid(B, L, K);
   if (fp64)
-    scatter_n_kernel<double><<<wgrid(tot), 256, 0, s>>>((const double2*)tmp, (double2*)flmn, B, N, L, n, L0);
+    scatter_slices_kernel<double><<<g, 256, 0, s>>>((const double2*)tmp, stride, (double2*)flmn, B, N,
+                                                    L, n0, K, L0);
   else
-    scatter_n_kernel<float><<<wgrid(tot), 256, 0, s>>>((const float2*)tmp, (float2*)flmn, B, N, L, n, L0);
+    scatter_slices_kernel<float><<<g, 256, 0, s>>>((const float2*)tmp, stride, (float2*)flmn, B, N, L,
+                                                   n0, K, L0);
   return cudaGetLastError();
 }
 
