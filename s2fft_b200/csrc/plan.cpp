@@ -1825,7 +1825,8 @@ static int run_pre_inverse(s2b_plan* p, const void* K, const void* flm, void* f,
   const int L = d.L;
   void* ftm = ws;
   const size_t ftm_bytes = (size_t)d.batch * p->nth * p->inv_ncol * 2 * p->rsz;
-  S2B_CK(cudaMemsetAsync(ftm, 0, ftm_bytes, s));
+  // (the tensor-core contraction writes every row of its columns)
+  if (!p->tc || p->kM != p->inv_ncol) S2B_CK(cudaMemsetAsync(ftm, 0, ftm_bytes, s));
   PreContractParams cp{};
   cp.L = L;
   cp.nth = p->nth;
@@ -1881,6 +1882,8 @@ static int run_pre_inverse(s2b_plan* p, const void* K, const void* flm, void* f,
   rp.phi0 = nullptr;  // the HEALPix phases are folded into the kernel table
   rp.tb = tables<Real>(p);
   rp.in = ftm;
+    tp.m0 = cp.mshift - (L - 1);
+    tp.rows_l = 0;
   rp.out = f;
   S2B_CK(launch_inv_rows<Real>(rp, p->nth, d.batch, p->maxM, s));
   return S2B_OK;
@@ -1939,7 +1942,8 @@ static int run_pre_forward(s2b_plan* p, const void* K, const void* f, void* flm,
     const int ncm = p->fwd_mode == 1 ? 2 * L - 1 : 2 * L;
     S2B_CK(launch_mw_cols<Real>(cp, ncm, d.batch, p->M1, p->M2, s));
   }
-  S2B_CK(cudaMemsetAsync(flm, 0, (size_t)d.batch * L * (2 * L - 1) * 2 * p->rsz, s));
+  if (!p->tc || p->kM != 2 * L - 1)
+    S2B_CK(cudaMemsetAsync(flm, 0, (size_t)d.batch * L * (2 * L - 1) * 2 * p->rsz, s));
   if (p->tc) {
     char* bp = raw + align256((size_t)d.batch * p->knth_fwd * p->kM * 2 * p->rsz);
     const int hpc = d.sampling == S2B_HEALPIX;
@@ -1983,6 +1987,8 @@ static int run_pre_forward(s2b_plan* p, const void* K, const void* f, void* flm,
 }
 
 // Adjoints of the precompute transforms (complex plans, float or double tables): the
+    tp.m0 = m0;
+    tp.rows_l = 1;
 // conjugate-transposed contraction with the same kernel table, composed with the adjoints
 // of the ring stages (unnormalised ring DFTs for the inverse; for the forward, inverse
 // ring DFTs and, on mw / mwss, the adjoint of the resampling chain in its raw form).

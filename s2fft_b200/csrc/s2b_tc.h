@@ -12,6 +12,8 @@ struct TcParams {
   int L, nth, M, B;
   int rows, kdim;         // output rows (l forward, t inverse) and summation length
   int cplx;               // complex kernel: K dimension doubled ([Re K | Im K])
+  int m0;                 // order m of column 0
+  int rows_l;             // 1: the rows are degrees (forward), 0: the summation index is (inverse)
   int nlt, ntc, nbg;      // filled by the launcher
   float sign;             // (-1)^s
   const __nv_bfloat16* Ap;  // packed kernel  [M][nlt][ntc][hi/lo][128 x 64]
@@ -34,6 +36,7 @@ cudaError_t launch_tc_pack_a(const float* K, int nth, int L, int M, int transpos
 // data element (map b, summation index q, column mi) at X[b in_map + q in_row + in_col0 + mi]
 cudaError_t launch_tc_pack_b(const void* X, int B, int kdim, int M, long in_map, int in_row,
                              int in_col0, int cplx, void* out, cudaStream_t s);
+// Writes every row of the M columns of every map (zeros where no degree reaches |m|).
 cudaError_t launch_tc_forward(TcParams p, cudaStream_t s);
 
 }  // namespace s2b
