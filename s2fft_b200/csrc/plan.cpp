@@ -1852,6 +1852,8 @@ static int run_pre_inverse(s2b_plan* p, const void* K, const void* flm, void* f,
     tp.B = d.batch;
     tp.rows = p->nth;
     tp.kdim = L;
+    tp.m0 = cp.mshift - (L - 1);
+    tp.rows_l = 0;
     tp.cplx = hpc;
     tp.sign = (float)cp.sign;
     tp.Ap = reinterpret_cast<const __nv_bfloat16*>(K);
@@ -1882,8 +1884,6 @@ static int run_pre_inverse(s2b_plan* p, const void* K, const void* flm, void* f,
   rp.phi0 = nullptr;  // the HEALPix phases are folded into the kernel table
   rp.tb = tables<Real>(p);
   rp.in = ftm;
-    tp.m0 = cp.mshift - (L - 1);
-    tp.rows_l = 0;
   rp.out = f;
   S2B_CK(launch_inv_rows<Real>(rp, p->nth, d.batch, p->maxM, s));
   return S2B_OK;
@@ -1956,6 +1956,8 @@ static int run_pre_forward(s2b_plan* p, const void* K, const void* f, void* flm,
     tp.B = d.batch;
     tp.rows = L;
     tp.kdim = p->knth_fwd;
+    tp.m0 = m0;
+    tp.rows_l = 1;
     tp.cplx = hpc;
     tp.out_map = (long)L * (2 * L - 1);
     tp.out_row = 2 * L - 1;
@@ -1987,8 +1989,6 @@ static int run_pre_forward(s2b_plan* p, const void* K, const void* f, void* flm,
 }
 
 // Adjoints of the precompute transforms (complex plans, float or double tables): the
-    tp.m0 = m0;
-    tp.rows_l = 1;
 // conjugate-transposed contraction with the same kernel table, composed with the adjoints
 // of the ring stages (unnormalised ring DFTs for the inverse; for the forward, inverse
 // ring DFTs and, on mw / mwss, the adjoint of the resampling chain in its raw form).
@@ -2339,6 +2339,14 @@ static int use_real_map_chain(s2b_plan* p) {
   return p->fwd_mode != 0 ? set_col_tables(p, true) : S2B_OK;
 }
 
+static void drop_aux(s2b_plan* p) {
+  if (p->aux) cudaStreamDestroy(p->aux);
+  if (p->aux_fork) cudaEventDestroy(p->aux_fork);
+  if (p->aux_join) cudaEventDestroy(p->aux_join);
+  p->aux = nullptr;
+  p->aux_fork = p->aux_join = nullptr;
+}
+
 static int build_wigner(s2b_plan* p) {
   const s2b_desc& d = p->d;
   p->fp64 = d.precision == S2B_F64;
@@ -2357,6 +2365,9 @@ static int build_wigner(s2b_plan* p) {
     int rc = s2b_plan_create(&sd, &sub);
     if (rc) return rc;
     p->subs.push_back(sub);
+    // the slices run side by side already: their low orders follow in the same stream instead
+    // of on a stream of their own (four event calls per slice and direction)
+    drop_aux(sub);
     // the slice n = 0 of a real signal is a real map: upstream transforms it as one
     // (wigner.py:521-530), so its MW / MWSS column chain takes the real-map corrections
     if (d.reality && n == 0 && (rc = use_real_map_chain(sub))) return rc;
@@ -2376,14 +2387,6 @@ static int build_wigner(s2b_plan* p) {
   return S2B_OK;
 }
 
-static void drop_aux(s2b_plan* p) {
-  if (p->aux) cudaStreamDestroy(p->aux);
-  if (p->aux_fork) cudaEventDestroy(p->aux_fork);
-  if (p->aux_join) cudaEventDestroy(p->aux_join);
-  p->aux = nullptr;
-  p->aux_fork = p->aux_join = nullptr;
-}
-
 // fban | per slice: coefficients | per stream: sub-transform workspace
 static size_t wigner_ws(const s2b_plan* p) {
   return align256(p->ws_w_fban) + p->subs.size() * align256(p->ws_w_tmp) +
@@ -2395,8 +2398,12 @@ static int run_wigner(s2b_plan* p, bool forward, const void* in, void* out, char
   const s2b_desc& d = p->d;
   const int n0 = d.reality ? 0 : -(d.N - 1);
   const int K = p->nwstream > 1 ? p->nwstream : 1;
+  const int nsub = (int)p->subs.size();
   char* fban = ws;
+  char* tmp = fban + align256(p->ws_w_fban);
+  char* sub_ws = tmp + nsub * align256(p->ws_w_tmp);
   const size_t slice = (size_t)d.batch * p->npix * 2 * p->rsz;
+  const long tstride = (long)(align256(p->ws_w_tmp) / (2 * p->rsz));
   int rc;
   if (forward)
     S2B_CK(launch_gamma_forward(p->fp64, in, fban, d.batch, d.N, p->npix, d.reality, s));
@@ -2405,9 +2412,6 @@ static int run_wigner(s2b_plan* p, bool forward, const void* in, void* out, char
   if (K > 1) {
     std::lock_guard<std::mutex> lk(p->fork_mu);
     S2B_CK(cudaEventRecord(p->wfork, s));
-    // the slices run side by side already: their low orders follow in the same stream instead
-    // of on a stream of their own (four event calls per slice and direction)
-    drop_aux(sub);
     for (int k = 0; k < K; ++k) S2B_CK(cudaStreamWaitEvent(p->wstream[k], p->wfork, 0));
   }
   rc = S2B_OK;
@@ -2430,12 +2434,8 @@ static int run_wigner(s2b_plan* p, bool forward, const void* in, void* out, char
       if (e != cudaSuccess && !rc) rc = fail(S2B_ERR_CUDA, std::string("Wigner join: ") + cudaGetErrorString(e));
     }
   }
-  const int nsub = (int)p->subs.size();
   if (rc) return rc;
-  char* tmp = fban + align256(p->ws_w_fban);
-  char* sub_ws = tmp + nsub * align256(p->ws_w_tmp);
   if (!forward) {
-  const long tstride = (long)(align256(p->ws_w_tmp) / (2 * p->rsz));
     S2B_CK(launch_gamma_inverse(p->fp64, fban, out, d.batch, d.N, p->npix, d.reality, s));
   } else {
     S2B_CK(launch_scatter_slices(p->fp64, tmp, tstride, out, d.batch, d.N, d.L, n0, nsub, d.L_lower, s));
