@@ -304,11 +304,22 @@ struct FFTBuild {
   int add(int n) {
     auto it = by_n.find(n);
     if (it != by_n.end()) return it->second;
+    const bool pow2 = (n & (n - 1)) == 0;
+    const int idx = make(n, pow2 ? n : (1 << ilog2(2 * n - 1)), !pow2, n);
+    maxM = std::max(maxM, descs[idx].M);
+    by_n[n] = idx;
+    return idx;
+  }
+
+  // Bluestein transform of length n whose inputs beyond the first nin are zero, on the working
+  // length M >= n + nin - 1
+  int add_bluestein(int n, int M, int nin) { return make(n, M, true, nin); }
+
+  int make(int n, int M, bool bluestein, int nin) {
     FFTDesc d{};
     d.n = n;
-    const bool pow2 = (n & (n - 1)) == 0;
-    d.bluestein = pow2 ? 0 : 1;
-    d.M = pow2 ? n : (1 << ilog2(2 * n - 1));
+    d.bluestein = bluestein ? 1 : 0;
+    d.M = M;
     if (d.M < 2) d.M = 2;
     d.logM = ilog2(d.M);
     auto tt = tw_by_M.find(d.M);
@@ -348,10 +359,8 @@ struct FFTBuild {
       }
       std::vector<cd> b(d.M, 0.0);
       b[0] = std::conj(w[0]);
-      for (int k = 1; k < n; ++k) {
-        b[k] = std::conj(w[k]);
-        b[d.M - k] = std::conj(w[k]);
-      }
+      for (int k = 1; k < n; ++k) b[k] = std::conj(w[k]);
+      for (int k = 1; k < nin; ++k) b[d.M - k] = std::conj(w[k]);
       fft_pow2_host(b);
       d.bf_off = (long)bf.size();
       std::vector<cd> br(d.M);
@@ -371,11 +380,8 @@ struct FFTBuild {
         rbf.insert(rbf.end(), rb.begin(), rb.end());
       }
     }
-    maxM = std::max(maxM, d.M);
-    const int idx = (int)descs.size();
     descs.push_back(d);
-    by_n[n] = idx;
-    return idx;
+    return (int)descs.size() - 1;
   }
 };
 
@@ -433,6 +439,10 @@ struct s2b_plan {
   void* rtw = nullptr;  // register-engine twiddles and filters
   void* rbf = nullptr;
   int row_desc = 0, col_d1 = 0, col_d2 = 0, maxM = 2, M1 = 2, M2 = 2;
+  // the forward column chain's transforms: on the register engine both work on Mreg points
+  // (col_f1, col_f2), else they are col_d1, col_d2 and Mreg = 0
+  int col_f1 = 0, col_f2 = 0, Mreg = 0;
+  bool col_pruned = false;
   void* col_ph = nullptr;  // column chain: chirp * half-sample phase / n1 per 4L-bin
   // start tables of the inverse rings (inverse and its adjoint), ring -> column map of the
   // adjoint spectra (recursed rings first, then north / south pole), adjoint chain table
@@ -983,6 +993,23 @@ static int build_plan(s2b_plan* p) {
     p->col_d2 = fb.add(4 * L);
     p->M1 = fb.descs[p->col_d1].M;
     p->M2 = fb.descs[p->col_d2].M;
+    // Register engine: one working length for both transforms. When 4L is a power of two, 4L
+    // (a theta length of 2L points then runs as Bluestein's, too). Else Bluestein's for both:
+    // the 4L-point transform has 2L inputs, so 6L - 1 points hold its convolution (8L - 1
+    // without that: half as many band-limits would need twice the length).
+    const int n1 = fb.descs[p->col_d1].n, n2 = 4 * L, top = p->fp64 ? 4096 : 8192;
+    p->col_f1 = p->col_d1;
+    p->col_f2 = p->col_d2;
+    p->col_pruned = (n2 & (n2 - 1)) != 0;
+    const int Mr = p->col_pruned ? 1 << ilog2(6 * L - 1) : n2;
+    // Short transforms have too few threads there (MW forward, float: L = 100 45 us against 38,
+    // L = 170 52 against 46; L = 200 53 and 53, L = 256 57 against 61, L = 301 74 against 94), and
+    // a theta length that is a power of two needs no Bluestein in the shared-memory passes.
+    if (L >= 192 && Mr <= top && (n1 & (n1 - 1)) != 0) {
+      p->Mreg = Mr;
+      if (p->M1 != Mr || !fb.descs[p->col_d1].bluestein) p->col_f1 = fb.add_bluestein(n1, Mr, n1);
+      if (p->col_pruned) p->col_f2 = fb.add_bluestein(n2, Mr, 2 * L);
+    }
   }
   p->maxM = 2;
   if (d.sampling == S2B_HEALPIX) {
@@ -1000,7 +1027,7 @@ static int build_plan(s2b_plan* p) {
     // factor applied to theta-DFT bin pp (stored at k = pp mod 4L) before the
     // inverse 4L DFT: Bluestein output chirp, MW half-sample shift exp(-i pp pi/(2L-1)),
     // and 1/n1
-    const FFTDesc& d1 = fb.descs[p->col_d1];
+    const FFTDesc& d1 = fb.descs[p->col_f1];
     const int n1 = d1.n, n2 = 4 * L;
     const int plo = p->fwd_mode == 1 ? -(L - 1) : -L, phi = L - 1;
     std::vector<cd> ph(n2, cd(0.0, 0.0));
@@ -1631,9 +1658,10 @@ static int fwd_stage_pre(s2b_plan* p, const void* f, char* ws, cudaStream_t s, F
     cp.TR = p->TR;
     cp.Gs = p->Gs;
     cp.scale = p->fwd_mode == 1 ? (2.0 * L) / (2.0 * L - 1.0) : 1.0;
-    cp.d1 = p->descs + p->col_d1;
-    cp.d2 = p->descs + p->col_d2;
-    cp.d2_pow2 = p->M2 == 4 * L;
+    cp.d1 = p->descs + p->col_f1;
+    cp.d2 = p->descs + p->col_f2;
+    cp.Mreg = p->Mreg;
+    cp.pruned = p->col_pruned;
     cp.ph = p->col_ph;
     cp.pole = p->col_pole;
     cp.imp = p->col_imp;
@@ -1928,9 +1956,10 @@ static int run_pre_forward(s2b_plan* p, const void* K, const void* f, void* flm,
     cp.M = p->kM;
     cp.m0 = m0;
     cp.scale = p->fwd_mode == 1 ? (2.0 * L) / (2.0 * L - 1.0) : 1.0;
-    cp.d1 = p->descs + p->col_d1;
-    cp.d2 = p->descs + p->col_d2;
-    cp.d2_pow2 = p->M2 == 4 * L;
+    cp.d1 = p->descs + p->col_f1;
+    cp.d2 = p->descs + p->col_f2;
+    cp.Mreg = p->Mreg;
+    cp.pruned = p->col_pruned;
     cp.ph = p->col_ph;
     cp.pole = p->col_pole;
     cp.imp = p->col_imp;

@@ -29,80 +29,6 @@
 
 namespace s2b {
 
-// CTAs per SM the register-engine kernels are compiled for (launch bounds): 32 warps per SM
-// in float (the points of a 2^LOGM transform take 2^(LOGM-4) threads; 64 registers, a few
-// bytes of spills at most), 16 in double (twice the registers per point); one CTA of 512
-// threads for 8192 points. The shared-memory passes (LOGM = 0): two in float, one in double.
-template <typename Real>
-__host__ __device__ constexpr int reg_min_blocks(int logm) {
-  // (registers are allocated per warp: a CTA of fewer than 32 threads counts as one warp;
-  // 256 points, whose 16 threads do the work of a warp, get half the warps per SM)
-  return logm == 0    ? (sizeof(Real) == 4 ? 2 : 1)
-         : logm >= 13 ? 1
-                      : (((sizeof(Real) == 4 ? 1024 : 512) >> (logm <= 8 ? 1 : 0)) >>
-                         (logm - 4 > 5 ? logm - 4 : 5));
-}
-
-// Any-length DFT of one CTA on the register engine (M = 2^LOGM, blockDim.x = M / 16; d.M
-// must be M): inputs load(k), k < d.n; every output X_k (k < d.n, conjugated when inv,
-// times the Bluestein output chirp unless chirp_out is false) goes to emit(k, X_k) once,
-// from the thread that holds it (natural order k = j + T a for Bluestein lengths, the
-// bit-reversed positions of a power-of-two length). buf: RegFFT<LOGM, NBUF>::SMEM_ELEMS
-// elements. With sync_emit a barrier precedes the emits, so that emit may write buf.
-template <typename Real, int LOGM, int NBUF, typename Load, typename Emit>
-__device__ __forceinline__ void reg_dft(typename C2<Real>::t* buf, const FFTDesc& d,
-                                        const FFTTables<Real>& tb, bool inv, bool chirp_out,
-                                        bool sync_emit, Load load, Emit emit) {
-  using R2 = typename C2<Real>::t;
-  using RF = RegFFT<LOGM, NBUF>;
-  const int j = threadIdx.x;
-  const R2* tw = tb.rtw + d.rtw_off;
-  int ping = 0;
-  R2 x[16];
-  if (d.bluestein) {
-    const R2* __restrict__ ch = tb.chirp + d.chirp_off;
-    const R2* __restrict__ bf = tb.rbf + d.rbf_off;  // position 16 j + a at [a T + j]
-    // the filter is read after the forward passes: its lines into L1 now, so that those
-    // reads do not wait on L2
-#pragma unroll
-    for (int a = 0; a < 16; ++a) prefetch_l1(bf + a * RF::T + j);
-#pragma unroll
-    for (int a = 0; a < 16; ++a) {
-      const int k = j + RF::T * a;
-      R2 v = czero<R2>();
-      if (k < d.n) {
-        v = load(k);
-        if (inv) v = cconj(v);
-        v = cmul(v, ch[k]);
-      }
-      x[a] = v;
-    }
-    RF::dif(x, buf, tw, false, ping);
-#pragma unroll
-    for (int a = 0; a < 16; ++a) x[a] = cmul(x[a], bf[a * RF::T + j]);
-    RF::dit(x, buf, tw, true, ping);
-    if (sync_emit) __syncthreads();
-#pragma unroll
-    for (int a = 0; a < 16; ++a) {
-      const int k = j + RF::T * a;
-      if (k < d.n) {
-        R2 v = chirp_out ? cmul(x[a], ch[k]) : x[a];
-        emit(k, inv ? cconj(v) : v);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int a = 0; a < 16; ++a) {
-      R2 v = load(j + RF::T * a);
-      x[a] = inv ? cconj(v) : v;
-    }
-    RF::dif(x, buf, tw, false, ping);
-    if (sync_emit) __syncthreads();
-#pragma unroll
-    for (int a = 0; a < 16; ++a) emit(bitrev(RF::point(j, a, 0), LOGM), inv ? cconj(x[a]) : x[a]);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Inverse rows: ftm [B][nrows][ncol] -> f (equiangular rows or HEALPix rings).
 // One CTA per (ring, map). Column c of ftm holds m = c - (L-1) - mo.
@@ -398,30 +324,48 @@ __global__ void __launch_bounds__(LOGM ? (1 << LOGM) / 16 : 512, reg_min_blocks<
 // The column chain's output for column m of map b: chain(t) = the inverse-DFT value on
 // MWSS(2L) ring t (t = 0..2L) with the pole and Nyquist corrections, before the overall
 // factor and the weights; writes it in the layout ColsParams describes (raw, ring pairs,
-// or rows), and the zero padding once per map (column m = 0).
-template <typename Real, typename Chain>
+// or rows). The zero padding of a map is spread over its 2L-1 columns: one CTA for all of it
+// was the tail of the whole launch (MW L = 128 forward: float 62 -> 48 us,
+// double 68 -> 56 us). Values are formed a few rings at a time before
+// they are stored, so that their loads do not wait for one another.
+// (U rings, for the shortest transforms: the long ones have warps enough and no registers to spare)
+template <int U, typename Real, typename Chain>
 __device__ __forceinline__ void cols_emit(const ColsParams<Real>& p, int b, int m, Chain chain) {
   using R2 = typename C2<Real>::t;
   const int L = p.L;
   const int nout = 2 * L + 1;
   const int am = m < 0 ? -m : m;
+  const int nt = blockDim.x;
   R2* out = reinterpret_cast<R2*>(p.out);
+  constexpr int UP = U > 1 ? U / 2 : 1;  // ring pairs
   if (p.raw) {
     if (m < p.m0) return;
-    for (int t = threadIdx.x; t < nout; t += blockDim.x) {
-      R2 u = chain(t);
-      u.x = (Real)((double)u.x * p.scale);
-      u.y = (Real)((double)u.y * p.scale);
-      out[((size_t)b * nout + t) * p.M + (m - p.m0)] = u;
+    for (int t0 = threadIdx.x; t0 < nout; t0 += U * nt) {
+      R2 u[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (t0 + k * nt < nout) u[k] = chain(t0 + k * nt);
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        const int t = t0 + k * nt;
+        if (t >= nout) break;
+        u[k].x = (Real)((double)u[k].x * p.scale);
+        u[k].y = (Real)((double)u[k].y * p.scale);
+        out[((size_t)b * nout + t) * p.M + (m - p.m0)] = u[k];
+      }
     }
     return;
   }
   auto weighted = [&](int t) -> R2 {
     R2 u = chain(t);
-    const double f = p.scale * p.weights[t];
+    const double f = p.scale * __ldg(p.weights + t);
     u.x = (Real)((double)u.x * f);
     u.y = (Real)((double)u.y * f);
     return u;
+  };
+  // this column's share of `total` pad entries
+  auto share = [&](int total, auto put) {
+    for (int x = (m + L - 1) * nt + (int)threadIdx.x; x < total; x += (2 * L - 1) * nt) put(x);
   };
   if (p.out2) {
     // ring pairs (t, 2L - t) as (E, O), in the layout of out with a trailing pair axis
@@ -431,18 +375,26 @@ __device__ __forceinline__ void cols_emit(const ColsParams<Real>& p, int b, int 
     const size_t rowbase =
         p.dual ? ((size_t)b * p.TR + mr) * p.Gs2 : ((size_t)b * p.nhalf * p.TR + mr) * p.Gs2;
     if (p.dual || m >= 0) {
-      for (int q = threadIdx.x; q < L; q += blockDim.x) {
-        const R2 un = weighted(q + 1);
-        R2 e = un, o = czero<R2>();
-        if (q < L - 1) {
-          const R2 us = weighted(2 * L - 1 - q);
-          e.x = un.x + us.x;
-          e.y = un.y + us.y;
-          o.x = un.x - us.x;
-          o.y = un.y - us.y;
+      for (int q0 = threadIdx.x; q0 < L; q0 += UP * nt) {
+        R2 un[UP], us[UP];
+#pragma unroll
+        for (int k = 0; k < UP; ++k) {
+          const int q = q0 + k * nt;
+          un[k] = q < L ? weighted(q + 1) : czero<R2>();
+          us[k] = q < L - 1 ? weighted(2 * L - 1 - q) : czero<R2>();
         }
-        o2[((rowbase + q) * 2 + 0) * per + (m < 0 ? 1 : 0)] = e;
-        o2[((rowbase + q) * 2 + 1) * per + (m < 0 ? 1 : 0)] = o;
+#pragma unroll
+        for (int k = 0; k < UP; ++k) {
+          const int q = q0 + k * nt;
+          if (q >= L) break;
+          R2 e = un[k], o = czero<R2>();
+          if (q < L - 1) {
+            e = cadd(un[k], us[k]);
+            o = csub(un[k], us[k]);
+          }
+          o2[((rowbase + q) * 2 + 0) * per + (m < 0 ? 1 : 0)] = e;
+          o2[((rowbase + q) * 2 + 1) * per + (m < 0 ? 1 : 0)] = o;
+        }
       }
     }
     // the pole rows stay in out (read by the epilogue)
@@ -455,77 +407,68 @@ __device__ __forceinline__ void cols_emit(const ColsParams<Real>& p, int b, int 
       else if (m >= 0)
         out[(((size_t)b * p.nhalf + 0) * p.TR + mr) * p.Gs + row] = u;
     }
-    if (m == 0) {
-      // zero pad rows (m outside [0, L)), pad pair columns (>= L) and, in the dual layout,
-      // the unused -m half of m = 0 (spin 0: one half)
-      const int rowlen = p.Gs2 * 2 * per;  // R2 entries per m row
-      R2* ob = o2 + (size_t)b * p.TR * rowlen;
-      for (int x = threadIdx.x; x < 2 * kPadLo * rowlen; x += blockDim.x) {
-        const int pr = x / rowlen;
-        const int mrow = pr < kPadLo ? pr : L + pr;
-        ob[(size_t)mrow * rowlen + x % rowlen] = czero<R2>();
-      }
-      const int padq = p.Gs2 - L;
-      for (int x = threadIdx.x; x < L * padq * 2 * per; x += blockDim.x) {
-        const int mrow = kPadLo + x / (padq * 2 * per);
-        ob[(size_t)mrow * rowlen + L * 2 * per + x % (padq * 2 * per)] = czero<R2>();
-      }
-      if (p.dual)
-        for (int x = threadIdx.x; x < L * 2; x += blockDim.x)
-          ob[(size_t)kPadLo * rowlen + x * 2 + 1] = czero<R2>();
-    }
+    // zero pad rows (m outside [0, L)), pad pair columns (>= L) and, in the dual layout,
+    // the unused -m half of m = 0 (spin 0: one half)
+    const int rowlen = p.Gs2 * 2 * per;  // R2 entries per m row
+    R2* ob = o2 + (size_t)b * p.TR * rowlen;
+    share(2 * kPadLo * rowlen, [&](int x) {
+      const int pr = x / rowlen;
+      const int mrow = pr < kPadLo ? pr : L + pr;
+      ob[(size_t)mrow * rowlen + x % rowlen] = czero<R2>();
+    });
+    const int padq = (p.Gs2 - L) * 2 * per;
+    share(L * padq, [&](int x) {
+      const int mrow = kPadLo + x / padq;
+      ob[(size_t)mrow * rowlen + L * 2 * per + x % padq] = czero<R2>();
+    });
+    if (p.dual)
+      share(L * 2, [&](int x) { ob[(size_t)kPadLo * rowlen + x * 2 + 1] = czero<R2>(); });
     return;
   }
-  for (int t = threadIdx.x; t < nout; t += blockDim.x) {
-    const R2 u = weighted(t);
-    const int row = t == 0 ? 2 * L - 1 : (t == 2 * L ? 2 * L : t - 1);  // poles after the recursed rings
-    const size_t mr = (size_t)(am + kPadLo);
-    if (p.dual) {
-      // Real4 {+m, -m} viewed as pairs of Real2
-      out[(((size_t)b * p.TR + mr) * p.Gs + row) * 2 + (m < 0 ? 1 : 0)] = u;
-    } else if (m >= 0) {
-      out[(((size_t)b * p.nhalf + 0) * p.TR + mr) * p.Gs + row] = u;
-    } else if (p.nhalf > 1) {
-      out[(((size_t)b * p.nhalf + 1) * p.TR + mr) * p.Gs + row] = u;
+  const int per = p.dual ? 2 : 1;  // dual: Real4 {+m, -m} viewed as pairs of Real2
+  const int halves = p.dual ? 1 : p.nhalf;
+  auto row_of = [&](int t) {  // poles after the recursed rings
+    return t == 0 ? 2 * L - 1 : (t == 2 * L ? 2 * L : t - 1);
+  };
+  const int half = p.dual || m >= 0 ? 0 : 1;
+  if (half < halves) {
+    R2* const orow = out + (((size_t)b * halves + half) * p.TR + am + kPadLo) * p.Gs * per +
+                     (p.dual && m < 0 ? 1 : 0);
+    for (int t0 = threadIdx.x; t0 < nout; t0 += U * nt) {
+      R2 u[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (t0 + k * nt < nout) u[k] = weighted(t0 + k * nt);
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (t0 + k * nt < nout) orow[(size_t)row_of(t0 + k * nt) * per] = u[k];
     }
   }
-  // zero pad rows (m outside [0, L)) and pad columns (>= 2L+1), once per map (m = 0 CTA)
-  if (m == 0) {
-    const int per = p.dual ? 2 : 1;
-    const int halves = p.dual ? 1 : p.nhalf;
-    const int padc = p.Gs - nout;
-    for (int x = threadIdx.x; x < halves * p.TR * padc * per; x += blockDim.x) {
-      const int c = x % (padc * per);
-      const int rowi = x / (padc * per);
-      out[(((size_t)b * halves * p.TR + rowi) * p.Gs + nout) * per + c] = czero<R2>();
-    }
-    for (int h = 0; h < halves; ++h)
-      for (int pr = 0; pr < 2 * kPadLo; ++pr) {
-        const int mr = pr < kPadLo ? pr : L + pr;  // rows m < 0 and m >= L
-        R2* base = out + (((size_t)b * halves + h) * p.TR + mr) * p.Gs * per;
-        for (int x = threadIdx.x; x < p.Gs * per; x += blockDim.x) base[x] = czero<R2>();
-      }
-    if (p.dual || p.nhalf > 1) {
-      // the unused half of m = 0 in the dual layout is zero as well
-      if (p.dual)
-        for (int t = threadIdx.x; t < nout; t += blockDim.x) {
-          const int row = t == 0 ? 2 * L - 1 : (t == 2 * L ? 2 * L : t - 1);
-          out[(((size_t)b * p.TR + kPadLo) * p.Gs + row) * 2 + 1] = czero<R2>();
-        }
-      else
-        for (int t = threadIdx.x; t < nout; t += blockDim.x) {
-          const int row = t == 0 ? 2 * L - 1 : (t == 2 * L ? 2 * L : t - 1);
-          out[(((size_t)b * p.nhalf + 1) * p.TR + kPadLo) * p.Gs + row] = czero<R2>();
-        }
-    }
-  }
+  // zero pad rows (m outside [0, L)) and pad columns (>= 2L+1)
+  R2* const ob = out + (size_t)b * halves * p.TR * p.Gs * per;
+  const int rowlen = p.Gs * per, padc = (p.Gs - nout) * per;
+  share(halves * p.TR * padc, [&](int x) {
+    ob[(size_t)(x / padc) * rowlen + nout * per + x % padc] = czero<R2>();
+  });
+  share(halves * 2 * kPadLo * rowlen, [&](int x) {
+    const int pr = x / rowlen, h = pr / (2 * kPadLo), r = pr % (2 * kPadLo);
+    const int mrow = r < kPadLo ? r : L + r;  // rows m < 0 and m >= L
+    ob[((size_t)h * p.TR + mrow) * rowlen + x % rowlen] = czero<R2>();
+  });
+  // the unused half of m = 0 (dual: its -m component) is zero as well
+  if (p.dual)
+    share(nout, [&](int t) {
+      ob[(size_t)kPadLo * rowlen + (size_t)row_of(t) * 2 + 1] = czero<R2>();
+    });
+  else if (halves > 1)
+    share(nout, [&](int t) {
+      ob[((size_t)p.TR + kPadLo) * rowlen + row_of(t)] = czero<R2>();
+    });
 }
 
-// LOGM > 0: both transforms on the register engine (d1.M = d2.M = 2^LOGM, the inverse DFT
-// of power-of-two length 4L; blockDim.x = 2^LOGM / 16); LOGM = 0: the shared-memory passes.
-template <typename Real, int LOGM, int NBUF>
-__global__ void __launch_bounds__(LOGM ? (1 << LOGM) / 16 : 512, reg_min_blocks<Real>(LOGM))
-    mw_cols_kernel(ColsParams<Real> p) {
+// The shared-memory passes, for working lengths beyond the register engine's.
+template <typename Real>
+__global__ void __launch_bounds__(512, reg_min_blocks<Real>(0)) mw_cols_kernel(ColsParams<Real> p) {
   chain_enter();
   using R2 = typename C2<Real>::t;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -535,8 +478,7 @@ __global__ void __launch_bounds__(LOGM ? (1 << LOGM) / 16 : 512, reg_min_blocks<
   // second are kept, phase-multiplied, in tmp in between
   R2* s1 = reinterpret_cast<R2*>(smem_raw);
   R2* s2 = s1;
-  R2* tmp = s1 + (LOGM > 0 ? RegFFT<(LOGM > 0 ? LOGM : 8), NBUF>::SMEM_ELEMS
-                           : padded_len(d1.M > d2.M ? d1.M : d2.M));
+  R2* tmp = s1 + padded_len(d1.M > d2.M ? d1.M : d2.M);
   const int L = p.L;
   const int mlo = p.mw ? -(L - 1) : -L;
   const int ncm = L - mlo;
@@ -560,19 +502,11 @@ __global__ void __launch_bounds__(LOGM ? (1 << LOGM) / 16 : 512, reg_min_blocks<
   const int phi = L - 1;
   const int n2 = d2.n;  // 4L
   const R2* __restrict__ ph = reinterpret_cast<const R2*>(p.ph);
-  if constexpr (LOGM > 0) {
-    // bin k of the theta DFT is p = k (k <= L-1) or k - n1; ph carries the Bluestein chirp
-    reg_dft<Real, LOGM, NBUF>(s1, d1, p.tb, false, false, false, load1, [&](int k, R2 v) {
-      const int pp = k <= phi ? k : k - n1;
-      if (pp >= plo) tmp[pp - plo] = cmul(v, ph[(pp + n2) % n2]);
-    });
-  } else {
-    dft_run<Real>(s1, d1, p.tb, false, load1);
-    for (int pp = plo + (int)threadIdx.x; pp <= phi; pp += blockDim.x) {
-      const int j = pmod(pp, n1);
-      const R2 g = d1.bluestein ? s1[pidx(j)] : s1[pidx(bitrev(j, d1.logM))];
-      tmp[pp - plo] = cmul(g, ph[(pp + n2) % n2]);
-    }
+  dft_run<Real>(s1, d1, p.tb, false, load1);
+  for (int pp = plo + (int)threadIdx.x; pp <= phi; pp += blockDim.x) {
+    const int j = pmod(pp, n1);
+    const R2 g = d1.bluestein ? s1[pidx(j)] : s1[pidx(bitrev(j, d1.logM))];
+    tmp[pp - plo] = cmul(g, ph[(pp + n2) % n2]);
   }
   __syncthreads();
   auto load2 = [&](int k) -> R2 {
@@ -585,21 +519,9 @@ __global__ void __launch_bounds__(LOGM ? (1 << LOGM) / 16 : 512, reg_min_blocks<
   const R2* __restrict__ pole = (p.mw && par) ? reinterpret_cast<const R2*>(p.pole) : nullptr;
   const R2 xpole = pole ? c[L - 1] : czero<R2>();
   const R2 nyq = (!p.mw && p.nyq_split) ? tmp[0] : czero<R2>();
-  if constexpr (LOGM > 0) {
-    // the 4L outputs in natural order in shared memory (after a barrier: the transform's
-    // last exchange may still be read)
-    reg_dft<Real, LOGM, NBUF>(s2, d2, p.tb, true, true, true, load2,
-                              [&](int k, R2 v) { s2[ridx(k)] = v; });
-    __syncthreads();
-  } else {
-    dft_run<Real>(s2, d2, p.tb, true, load2);
-  }
+  dft_run<Real>(s2, d2, p.tb, true, load2);
   auto chain = [&](int t) -> R2 {
-    R2 u;
-    if constexpr (LOGM > 0)
-      u = s2[ridx(t)];
-    else
-      u = dft_get<Real>(s2, d2, p.tb, true, t);
+    R2 u = dft_get<Real>(s2, d2, p.tb, true, t);
     if (pole) u = cadd(u, cmul(xpole, pole[t]));
     if (t & 1) {  // i N sin(pi t / 2)
       const Real sg = (t & 2) ? Real(-1) : Real(1);
@@ -608,7 +530,7 @@ __global__ void __launch_bounds__(LOGM ? (1 << LOGM) / 16 : 512, reg_min_blocks<
     }
     return u;
   };
-  cols_emit(p, b, m, chain);
+  cols_emit<1>(p, b, m, chain);
 }
 
 // Two columns per CTA on the register engine: m and m + 1 have opposite parities
@@ -624,6 +546,9 @@ __global__ void __launch_bounds__(LOGM ? (1 << LOGM) / 16 : 512, reg_min_blocks<
 //   * MWSS: the theta-Nyquist bin p = -L, which only the even column has (u gets
 //     N (-i)^t, and the split correction for real maps).
 // The last column of the odd count 2L-1 runs alone (x_B = 0).
+// Both transforms share one working length 2^LOGM (FFTDescs of the plan) of up to 8192 points
+// (4096 in double). Against the shared-memory passes, one column at a time: MW L = 700 float
+// forward 356 -> 269 us, L = 301 double 140 -> 90 us.
 template <typename Real, int LOGM, int NBUF>
 __global__ void __launch_bounds__((1 << LOGM) / 16, reg_min_blocks<Real>(LOGM))
     mw_cols_pair_kernel(ColsParams<Real> p) {
@@ -676,15 +601,34 @@ __global__ void __launch_bounds__((1 << LOGM) / 16, reg_min_blocks<Real>(LOGM))
   __syncthreads();
   // MWSS: the Nyquist bin (tmp[0]) belongs to the even column alone
   const R2 nyqZ = p.mw ? czero<R2>() : tmp[0];
+  // pruned: the bins p = -L .. L-1 come first, so the output t carries exp(2 pi i t (-L) / 4L)
+  // = (-i)^t
+  const bool pruned = p.pruned != 0;
   auto load2 = [&](int k) -> R2 {
-    const int pp = k <= phi ? k : k - n2;
+    const int pp = pruned ? k - L : k <= phi ? k : k - n2;
     return (pp < plo || pp > phi || (!p.mw && pp == -L)) ? czero<R2>() : tmp[pp - plo];
   };
-  reg_dft<Real, LOGM, NBUF>(s, d2, p.tb, true, true, true, load2,
-                            [&](int k, R2 v) { s[ridx(k)] = v; });
+  reg_dft<Real, LOGM, NBUF>(s, d2, p.tb, true, true, true, load2, [&](int k, R2 v) {
+    if (pruned) {
+      if (k & 2) v = cscale(v, Real(-1));
+      if (k & 1) {  // times -i
+        const Real x = v.x;
+        v.x = v.y;
+        v.y = -x;
+      }
+    }
+    s[ridx(k)] = v;
+  });
   __syncthreads();
   const R2* __restrict__ imp = reinterpret_cast<const R2*>(p.imp);
   const int nout = 2 * L + 1;
+  // the odd column's self-mirrored samples
+  R2 self0 = czero<R2>(), self1 = czero<R2>();
+  if (oddA || hasB) {
+    const R2* c = oddA ? cA : cB;
+    self0 = c[p.mw ? L - 1 : 0];
+    if (!p.mw) self1 = c[L];
+  }
   // column A (B): sym = +1 (-1) picks u_A (u_B) out of z'
   auto chain = [&](bool colA, int t) -> R2 {
     const R2 zp = s[ridx(t)], zm = s[ridx(t == 0 ? 0 : n2 - t)];
@@ -697,14 +641,9 @@ __global__ void __launch_bounds__((1 << LOGM) / 16, reg_min_blocks<Real>(LOGM))
       u.y = -d.x;
     }
     const bool odd = colA == oddA;
-    const R2* c = colA ? cA : cB;
     if (odd) {
-      if (p.mw) {
-        u = cadd(u, cmul(c[L - 1], imp[t]));
-      } else {
-        u = cadd(u, cmul(c[0], imp[t]));
-        u = cadd(u, cmul(c[L], imp[nout + t]));
-      }
+      u = cadd(u, cmul(self0, imp[t]));
+      if (!p.mw) u = cadd(u, cmul(self1, imp[nout + t]));
     } else if (!p.mw) {
       // N (-i)^t from the Nyquist bin, N = the even column's bin -L
       R2 N = nyqZ;
@@ -728,8 +667,9 @@ __global__ void __launch_bounds__((1 << LOGM) / 16, reg_min_blocks<Real>(LOGM))
     }
     return u;
   };
-  cols_emit(p, b, mA, [&](int t) { return chain(true, t); });
-  if (hasB) cols_emit(p, b, mA + 1, [&](int t) { return chain(false, t); });
+  constexpr int U = LOGM <= 10 ? 4 : 1;
+  cols_emit<U>(p, b, mA, [&](int t) { return chain(true, t); });
+  if (hasB) cols_emit<U>(p, b, mA + 1, [&](int t) { return chain(false, t); });
 }
 
 // ---------------------------------------------------------------------------
@@ -849,9 +789,7 @@ static constexpr int kRegBufs = 1;  // exchange buffers of the register engine
 template <typename Real, typename Kernel, typename Params>
 static cudaError_t launch_fft_kernel(Kernel k, dim3 grid, int threads, size_t smem,
                                      const Params& p, cudaStream_t s, int carveout = 100) {
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
+  const cudaError_t e = func_limits(k, smem, carveout);
   if (e != cudaSuccess) return e;
   return launch_chained(k, grid, dim3(threads), smem, s, p);
 }
@@ -928,34 +866,21 @@ cudaError_t launch_mw_cols(const ColsParams<Real>& p, int ncm, int batch, int M1
                            cudaStream_t s) {
   using R2 = typename C2<Real>::t;
   const dim3 grid(ncm, batch);
-  // register engine: one working length for both transforms, the second a plain power of two
-  const int lg = (M1 == M2 && p.d2_pow2) ? reg_logm<Real>(M1) : 0;
   const int extra = 2 * p.L;
-  if (p.imp) {
+  if (p.Mreg) {
     // columns m, m+1 per CTA: L CTAs per map cover m = -(L-1) .. L-1
     const dim3 gp(p.L, batch);
-    switch (lg) {
-      case 8: return launch_fft_kernel<Real>(mw_cols_pair_kernel<Real, 8, kRegBufs>, gp, 16, reg_smem<Real, 8>(extra), p, s, reg_carveout<Real, 8>(extra));
-      case 9: return launch_fft_kernel<Real>(mw_cols_pair_kernel<Real, 9, kRegBufs>, gp, 32, reg_smem<Real, 9>(extra), p, s, reg_carveout<Real, 9>(extra));
+    switch (reg_logm<Real>(p.Mreg)) {
       case 10: return launch_fft_kernel<Real>(mw_cols_pair_kernel<Real, 10, kRegBufs>, gp, 64, reg_smem<Real, 10>(extra), p, s, reg_carveout<Real, 10>(extra));
       case 11: return launch_fft_kernel<Real>(mw_cols_pair_kernel<Real, 11, kRegBufs>, gp, 128, reg_smem<Real, 11>(extra), p, s, reg_carveout<Real, 11>(extra));
       case 12: return launch_fft_kernel<Real>(mw_cols_pair_kernel<Real, 12, kRegBufs>, gp, 256, reg_smem<Real, 12>(extra), p, s, reg_carveout<Real, 12>(extra));
       case 13: return launch_fft_kernel<Real>(mw_cols_pair_kernel<Real, 13, kRegBufs>, gp, 512, reg_smem<Real, 13>(extra), p, s, reg_carveout<Real, 13>(extra));
-      default: break;
+      default: return cudaErrorInvalidValue;
     }
-  }
-  switch (lg) {
-    case 8: return launch_fft_kernel<Real>(mw_cols_kernel<Real, 8, kRegBufs>, grid, 16, reg_smem<Real, 8>(extra), p, s, reg_carveout<Real, 8>(extra));
-    case 9: return launch_fft_kernel<Real>(mw_cols_kernel<Real, 9, kRegBufs>, grid, 32, reg_smem<Real, 9>(extra), p, s, reg_carveout<Real, 9>(extra));
-    case 10: return launch_fft_kernel<Real>(mw_cols_kernel<Real, 10, kRegBufs>, grid, 64, reg_smem<Real, 10>(extra), p, s, reg_carveout<Real, 10>(extra));
-    case 11: return launch_fft_kernel<Real>(mw_cols_kernel<Real, 11, kRegBufs>, grid, 128, reg_smem<Real, 11>(extra), p, s, reg_carveout<Real, 11>(extra));
-    case 12: return launch_fft_kernel<Real>(mw_cols_kernel<Real, 12, kRegBufs>, grid, 256, reg_smem<Real, 12>(extra), p, s, reg_carveout<Real, 12>(extra));
-    case 13: return launch_fft_kernel<Real>(mw_cols_kernel<Real, 13, kRegBufs>, grid, 512, reg_smem<Real, 13>(extra), p, s, reg_carveout<Real, 13>(extra));
-    default: break;
   }
   // one DFT buffer plus the 2L bins carried between the two transforms
   const size_t smem = (size_t)(padded_len(M1 > M2 ? M1 : M2) + 2 * p.L) * sizeof(R2);
-  return launch_fft_kernel<Real>(mw_cols_kernel<Real, 0, 1>, grid, fft_threads(M1 > M2 ? M1 : M2),
+  return launch_fft_kernel<Real>(mw_cols_kernel<Real>, grid, fft_threads(M1 > M2 ? M1 : M2),
                                  smem, p, s);
 }
 

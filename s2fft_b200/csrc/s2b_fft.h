@@ -79,7 +79,8 @@ struct ColsParams {
   double scale;         // overall factor of the chain
   const FFTDesc* d1;    // theta DFT over the periodic extension (2L-1 or 2L)
   const FFTDesc* d2;    // inverse DFT of length 4L
-  int d2_pow2;          // 4L is a power of two (d2 without Bluestein)
+  int Mreg;             // working length of d1 and d2 on the register engine (0: not used)
+  int pruned;           // register engine, d2: Bluestein's of the 2L bins from p = -L on
   const double* weights;// 2L+1 MWSS(2L) transform weights
   const void* ph;       // [4L] complex factor of theta-DFT bin p (at p mod 4L), 0 outside
   const void* ph_adj;   // [4L] adjoint chain: conj(half-sample phase) / n1 (at p mod 4L)
@@ -89,8 +90,8 @@ struct ColsParams {
   // the chain's response (before scale and weights) to a unit impulse on the samples that are
   // their own mirror in the theta extension, for columns with odd m + s: MW [2L+1] (the pole
   // ring t = L-1, pole correction included), MWSS [2][2L+1] (t = 0, t = L; Nyquist split
-  // included). Set: the register engine transforms two columns per CTA
-  // (mw_cols_pair_kernel); nullptr: one column per CTA
+  // included); used by the register engine, which transforms two columns per CTA
+  // (mw_cols_pair_kernel)
   const void* imp;
   // MWSS real maps: the theta-Nyquist bin N (p = -L) counts half at -L and half at +L, i.e.
   // i N sin(pi k / 2) is added to the output on ring k

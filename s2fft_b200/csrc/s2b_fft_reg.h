@@ -24,6 +24,7 @@
 
 #include <cuda_runtime.h>
 
+#include "s2b_dev.h"
 #include "s2b_fft_dev.h"
 
 namespace s2b {
@@ -229,5 +230,79 @@ struct RegFFT {
     for (int g = 0; g < G; ++g) reg_stage<NS0, false, G, 0>(x + g, b0[g], inv);
   }
 };
+
+// CTAs per SM the register-engine kernels are compiled for (launch bounds): 32 warps per SM
+// in float (the points of a 2^LOGM transform take 2^(LOGM-4) threads; 64 registers, a few
+// bytes of spills at most), 16 in double (twice the registers per point); one CTA of 512
+// threads for 8192 points. The shared-memory passes (LOGM = 0): two in float, one in double.
+template <typename Real>
+__host__ __device__ constexpr int reg_min_blocks(int logm) {
+  // (registers are allocated per warp: a CTA of fewer than 32 threads counts as one warp;
+  // 256 points, whose 16 threads do the work of a warp, get half the warps per SM)
+  return logm == 0    ? (sizeof(Real) == 4 ? 2 : 1)
+         : logm >= 13 ? 1
+                      : (((sizeof(Real) == 4 ? 1024 : 512) >> (logm <= 8 ? 1 : 0)) >>
+                         (logm - 4 > 5 ? logm - 4 : 5));
+}
+
+// Any-length DFT of one CTA on the register engine (M = 2^LOGM, blockDim.x = M / 16; d.M
+// must be M): inputs load(k), k < d.n; every output X_k (k < d.n, conjugated when inv,
+// times the Bluestein output chirp unless chirp_out is false) goes to emit(k, X_k) once,
+// from the thread that holds it (natural order k = j + T a for Bluestein lengths, the
+// bit-reversed positions of a power-of-two length). buf: RegFFT<LOGM, NBUF>::SMEM_ELEMS
+// elements. With sync_emit a barrier precedes the emits, so that emit may write buf.
+template <typename Real, int LOGM, int NBUF, typename Load, typename Emit>
+__device__ __forceinline__ void reg_dft(typename C2<Real>::t* buf, const FFTDesc& d,
+                                        const FFTTables<Real>& tb, bool inv, bool chirp_out,
+                                        bool sync_emit, Load load, Emit emit) {
+  using R2 = typename C2<Real>::t;
+  using RF = RegFFT<LOGM, NBUF>;
+  const int j = threadIdx.x;
+  const R2* tw = tb.rtw + d.rtw_off;
+  int ping = 0;
+  R2 x[16];
+  if (d.bluestein) {
+    const R2* __restrict__ ch = tb.chirp + d.chirp_off;
+    const R2* __restrict__ bf = tb.rbf + d.rbf_off;  // position 16 j + a at [a T + j]
+    // the filter is read after the forward passes: its lines into L1 now, so that those
+    // reads do not wait on L2
+#pragma unroll
+    for (int a = 0; a < 16; ++a) prefetch_l1(bf + a * RF::T + j);
+#pragma unroll
+    for (int a = 0; a < 16; ++a) {
+      const int k = j + RF::T * a;
+      R2 v = czero<R2>();
+      if (k < d.n) {
+        v = load(k);
+        if (inv) v = cconj(v);
+        v = cmul(v, ch[k]);
+      }
+      x[a] = v;
+    }
+    RF::dif(x, buf, tw, false, ping);
+#pragma unroll
+    for (int a = 0; a < 16; ++a) x[a] = cmul(x[a], bf[a * RF::T + j]);
+    RF::dit(x, buf, tw, true, ping);
+    if (sync_emit) __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 16; ++a) {
+      const int k = j + RF::T * a;
+      if (k < d.n) {
+        R2 v = chirp_out ? cmul(x[a], ch[k]) : x[a];
+        emit(k, inv ? cconj(v) : v);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int a = 0; a < 16; ++a) {
+      R2 v = load(j + RF::T * a);
+      x[a] = inv ? cconj(v) : v;
+    }
+    RF::dif(x, buf, tw, false, ping);
+    if (sync_emit) __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 16; ++a) emit(bitrev(RF::point(j, a, 0), LOGM), inv ? cconj(x[a]) : x[a]);
+  }
+}
 
 }  // namespace s2b

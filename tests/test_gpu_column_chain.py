@@ -1,0 +1,47 @@
+"""The MW / MWSS column chain at the band-limits where its transforms change: the shared-memory
+passes up to L = 191, the register engine from there on, 4L a power of two, 6L - 1 against the
+powers of two, and the largest working lengths with the first band-limit beyond."""
+
+import numpy as np
+import pytest
+
+import oracle
+from tests.conftest import relerr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def s2b():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import s2fft_b200
+
+    return s2fft_b200
+
+
+@pytest.mark.parametrize("sampling", ["mw", "mwss"])
+@pytest.mark.parametrize("L", [2, 3, 16, 64, 85, 128, 191, 192, 193, 256])
+@pytest.mark.parametrize("spin,reality", [(0, False), (1, False), (0, True)])
+def test_forward_against_oracle(s2b, rng, sampling, L, spin, reality):
+    """White noise on the grid: both parities, the self-mirrored samples and the Nyquist bin
+    count (tolerances: the float64 path's and float32 path's bounds on the whole transform)."""
+    shape = s2b.spherical.f_shape(L, sampling)
+    f = rng.standard_normal(shape) + (0 if reality else 1j * rng.standard_normal(shape))
+    ref = oracle.spherical.forward(f, L, spin, None, sampling, reality=reality, backend="c")
+    for precision, tol in (("f64", 1e-10), ("f32", 1e-5)):
+        y = s2b.forward(f, L, spin, None, sampling, reality=reality, precision=precision)
+        assert relerr(y, ref) < tol, (precision, relerr(y, ref))
+
+
+@pytest.mark.parametrize("sampling", ["mw", "mwss"])
+@pytest.mark.parametrize("precision,L", [("f64", 341), ("f64", 342), ("f64", 682), ("f64", 683),
+                                         ("f32", 682), ("f32", 683), ("f32", 1365),
+                                         ("f32", 1366)])
+def test_round_trip_at_the_length_limits(s2b, rng, sampling, precision, L):
+    flm = oracle.signal.generate_flm(rng, L, 0, 0, False)
+    f = s2b.inverse(flm, L, 0, None, sampling, precision=precision)
+    y = s2b.forward(f, L, 0, None, sampling, precision=precision)
+    assert relerr(y, flm) < (1e-10 if precision == "f64" else 1e-5), relerr(y, flm)
