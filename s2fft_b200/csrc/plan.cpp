@@ -2507,7 +2507,7 @@ static int upload_complex_to(std::vector<void*>* allocs, bool fp64, void** dst,
 }
 
 int s2b::build_fft_set(const int* lengths, int count, bool fp64, std::vector<void*>* allocs,
-                       FFTSet* out) {
+                       FFTSet* out, int blu_n, int blu_M) {
   FFTBuild fb;
   out->host.clear();
   std::vector<int> idx(count);
@@ -2515,11 +2515,14 @@ int s2b::build_fft_set(const int* lengths, int count, bool fp64, std::vector<voi
     if (lengths[i] < 2) return fail(S2B_ERR_INVALID, "FFT length must be >= 2");
     idx[i] = fb.add(lengths[i]);
   }
-  for (int i = 0; i < count; ++i) out->host.push_back(fb.descs[idx[i]]);
+  if (blu_n > 0) idx.push_back(fb.add_bluestein(blu_n, blu_M, blu_n));
+  for (int i : idx) out->host.push_back(fb.descs[i]);
   int rc;
   if ((rc = upload_complex_to(allocs, fp64, &out->tw, fb.tw))) return rc;
   if ((rc = upload_complex_to(allocs, fp64, &out->chirp, fb.chirp))) return rc;
   if ((rc = upload_complex_to(allocs, fp64, &out->bf, fb.bf))) return rc;
+  if ((rc = upload_complex_to(allocs, fp64, &out->rtw, fb.rtw))) return rc;
+  if ((rc = upload_complex_to(allocs, fp64, &out->rbf, fb.rbf))) return rc;
   return S2B_OK;
 }
 

@@ -38,11 +38,14 @@ struct FFTSet {
   void* tw = nullptr;
   void* chirp = nullptr;
   void* bf = nullptr;
+  void* rtw = nullptr;  // register engine
+  void* rbf = nullptr;
 };
 // Builds the set for `count` lengths (each >= 2) in float or double; every device
-// allocation is appended to *allocs (the caller frees them).
+// allocation is appended to *allocs (the caller frees them). blu_n > 0: one more descriptor
+// at the end, Bluestein's for length blu_n on the working length blu_M.
 int build_fft_set(const int* lengths, int count, bool fp64, std::vector<void*>* allocs,
-                  FFTSet* out);
+                  FFTSet* out, int blu_n = 0, int blu_M = 0);
 
 // Records msg as the calling thread's s2b_last_error() text and returns code.
 int set_last_error(int code, const char* msg);
