@@ -1459,6 +1459,11 @@ static int run_inverse_adjoint(s2b_plan* p, const void* gf, void* gflm, char* ws
     lp.NB = p->fwd_NB;
     lp.Mst = p->inv_Mst;
     lp.Vst = p->inv_Vst;
+    // the m-split of the inverse on the same rings: one segment leaves 256 CTAs at L = 1024
+    // (float MW L = 1024 loss and gradient 913 -> 669 us)
+    lp.Mst1 = p->inv_Mst1;
+    lp.Vst1 = p->inv_Vst1;
+    lp.nseg = p->inv_nseg;
     lp.Hb = p->fwd_Hb;
     lp.lam = p->inv_lam;
     lp.Ls = p->inv_Ls;
