@@ -56,15 +56,50 @@ struct Inv2Layout {
   // use different halves, so one barrier per group separates them
   // (once when two copies would leave room for fewer than 3 CTAs per SM: then a second
   // barrier per group)
-  static constexpr int buf_elems = R * W * NRT * NE;
+  // The sums lie in pieces of at most 16 bytes (a double4 is two) with a warp's lanes side by
+  // side, ring lane * T + i at i * 32 + lane, so that a store fills whole wavefronts; a step's
+  // pieces are padded so that the reduction's lanes (the R steps of a ring next to one another)
+  // read different banks.
+  using Piece = std::conditional_t<sizeof(Acc) == 32, typename Vec<Real>::t2, Acc>;
+  static constexpr int NP = (int)(sizeof(Acc) / sizeof(Piece));
+  static constexpr int piece_elems = W * NRT;  // and O follows E by NP * piece_elems
+  static constexpr int step_elems = NE * NP * piece_elems + 16 / (int)sizeof(Piece);
+  static constexpr int buf_elems = R * step_elems;
+  __device__ __forceinline__ static void put(Piece* e, const Acc& a) {
+    if constexpr (NP == 1) {
+      *e = a;
+    } else {
+      Piece u;
+      u.x = a.x;
+      u.y = a.y;
+      e[0] = u;
+      u.x = a.z;
+      u.y = a.w;
+      e[piece_elems] = u;
+    }
+  }
+  __device__ __forceinline__ static Acc get(const Piece* e) {
+    if constexpr (NP == 1) {
+      return *e;
+    } else {
+      const Piece u = e[0], v = e[piece_elems];
+      Acc a;
+      a.x = u.x;
+      a.y = u.y;
+      a.z = v.x;
+      a.w = v.y;
+      return a;
+    }
+  }
   // start values of the CTA's states: [2 blocks][NRT rings][32] (d~_M, d~_{M+1})
   // (VST: staged by bulk copy; otherwise each lane reads its own from global memory, which
   // leaves room for one more CTA per SM)
   static constexpr size_t v_bytes = VST ? (size_t)2 * NRT * kFwdBlock * 2 * sizeof(Real) : 0;
-  static constexpr size_t fixed_bytes = 2 * stage_bytes + v_bytes + 32;
+  static constexpr size_t row_bytes = 2 * NRT * sizeof(int);  // ftm rows of the rings, mirrors
+  static constexpr size_t fixed_bytes = 2 * stage_bytes + v_bytes + 32 + row_bytes;
   static constexpr int NBUF =
-      3 * (fixed_bytes + 2 * buf_elems * sizeof(Acc) + 1024) <= 228 * 1024 ? 2 : 1;
-  static constexpr size_t buf_bytes = (size_t)NBUF * buf_elems * sizeof(Acc);
+      3 * (fixed_bytes + 2 * buf_elems * sizeof(Piece) + 1024) <= 228 * 1024 ? 2 : 1;
+  static constexpr size_t buf_bytes = (size_t)NBUF * buf_elems * sizeof(Piece);
   static constexpr size_t total = fixed_bytes + buf_bytes;
   static_assert(W == 4, "two warps per 32-degree block, two blocks per CTA");
   static_assert(stage_bytes % 16 == 0 && buf_bytes % 16 == 0, "align");
@@ -100,7 +135,6 @@ template <typename Real, bool DUAL, int T, int W, int R, bool VST, bool SYM>
 __device__ __forceinline__ bool lat_inv2_tile(const Inv2Params& p, int bx, int by, int bz,
                                               unsigned char* smem_raw, bool& live) {
   using Lay = Inv2Layout<Real, DUAL, T, W, R, VST, SYM>;
-  constexpr int NE = Lay::NE;
   using Acc = typename Lay::Acc;
   using R2 = typename Vec<Real>::t2;
   constexpr int K = Lay::K;
@@ -108,7 +142,8 @@ __device__ __forceinline__ bool lat_inv2_tile(const Inv2Params& p, int bx, int b
   constexpr int NT = Lay::NT;
   static_assert(R == 4 || R == 8, "the group body below is written for R = 4 or 8");
   unsigned char* stage_base = smem_raw;
-  Acc* const bufs = reinterpret_cast<Acc*>(smem_raw + 2 * Lay::stage_bytes);
+  using Piece = typename Lay::Piece;
+  Piece* const bufs = reinterpret_cast<Piece*>(smem_raw + 2 * Lay::stage_bytes);
   const typename Vec<Real>::t2* vS = reinterpret_cast<const typename Vec<Real>::t2*>(
       smem_raw + 2 * Lay::stage_bytes + Lay::buf_bytes);
   uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + 2 * Lay::stage_bytes + Lay::buf_bytes +
@@ -237,19 +272,12 @@ __device__ __forceinline__ bool lat_inv2_tile(const Inv2Params& p, int bx, int b
     lmax = kb1 * kFwdBlock + kFwdBlock - 1;
   if (lmax > L - 1) lmax = L - 1;
 
-  // the reduction gives every thread one ring of the tile (NT is a multiple of NRT): its
-  // ftm rows (and, symmetric, its mirror's), looked up once
-  static_assert(NT % NRT == 0, "one reduction ring per thread");
-  const int rr_red = tid % NRT;
-  const int r_red = r0 + rr_red;
-  const bool ring_live = r_red < p.nrings;
-  R2* ftm_r = nullptr;
-  R2* ftm_rm = nullptr;  // symmetric: the mirror ring (none for the equator)
-  if (ring_live) {
-    ftm_r = reinterpret_cast<R2*>(p.ftm) + ((size_t)b * p.nrows + p.ring_row[r_red]) * p.ncol;
-    if (SYM && RS - 1 - r_red != r_red)
-      ftm_rm = reinterpret_cast<R2*>(p.ftm) +
-               ((size_t)b * p.nrows + p.ring_row[RS - 1 - r_red]) * p.ncol;
+  // ftm rows of the tile's rings (and, symmetric, of their mirrors: none for the equator)
+  int* const rowS = reinterpret_cast<int*>(mbar + 4);
+  for (int i = tid; i < NRT; i += NT) {
+    const int r = r0 + i;
+    rowS[i] = r < p.nrings ? p.ring_row[r] : -1;
+    rowS[NRT + i] = SYM && r < p.nrings && RS - 1 - r != r ? p.ring_row[RS - 1 - r] : -1;
   }
   // start values read from global memory: each lane's line is prefetched into L1 one group
   // before the group that starts the state (a group is thousands of cycles of FMAs)
@@ -290,7 +318,7 @@ __device__ __forceinline__ bool lat_inv2_tile(const Inv2Params& p, int bx, int b
           }
         }
     const unsigned char* st = stage_base + (size_t)(grp & 1) * Lay::stage_bytes;
-    Acc* const buf = bufs + (Lay::NBUF == 2 ? (grp & 1) * Lay::buf_elems : 0);
+    Piece* const buf = bufs + (Lay::NBUF == 2 ? (grp & 1) * Lay::buf_elems : 0);
     const Real* hS = reinterpret_cast<const Real*>(st) + col0;
     const Acc* fS = reinterpret_cast<const Acc*>(st + Lay::h_bytes) + col0;
     const Real* lS = reinterpret_cast<const Real*>(st + Lay::h_bytes + Lay::f_bytes) + lane * T;
@@ -330,12 +358,12 @@ __device__ __forceinline__ bool lat_inv2_tile(const Inv2Params& p, int bx, int b
       if constexpr (SYM) {                                                              \
         /* l = 32 block + 8 warp + kk: l + m even for kk = m mod 2 */                   \
         const int pe = m & 1;                                                           \
-        Acc* e = buf + (((S) * W + wp) * NRT + lane * T + i) * 2;                       \
-        e[0] = pe ? a[1][i] : a[0][i];                                                  \
-        e[1] = pe ? a[0][i] : a[1][i];                                                  \
+        Piece* e = buf + (S) * Lay::step_elems + wp * NRT + i * 32 + lane;              \
+        Lay::put(e, pe ? a[1][i] : a[0][i]);                                            \
+        Lay::put(e + Lay::NP * Lay::piece_elems, pe ? a[0][i] : a[1][i]);               \
       } else {                                                                          \
         acc_add(a[0][i], a[1][i]);                                                      \
-        buf[((S) * W + wp) * NRT + lane * T + i] = a[0][i];                             \
+        Lay::put(buf + (S) * Lay::step_elems + wp * NRT + i * 32 + lane, a[0][i]);      \
       }                                                                                 \
     }                                                                                   \
   }
@@ -360,36 +388,47 @@ __device__ __forceinline__ bool lat_inv2_tile(const Inv2Params& p, int bx, int b
     }
     // every warp is past this group's stage: refill it for group grp + 2
     if (tid == 0 && grp + 2 < ngroups) issue(grp + 2);
-    // warps' partial sums -> ring spectra (NT is a multiple of NRT: one ring per thread)
+    // warps' partial sums -> ring spectra. The R orders of a ring are neighbours in its
+    // spectrum, so they go to neighbouring lanes: a warp's atomics cover 32 / R rows in runs
+    // of R entries instead of 32 rows.
     for (int it = tid; it < R * NRT; it += NT) {
-      const int S = it / NRT;
-      const int m = mgrp - S;
-      if (m < p.mlo || m > lmax || !ring_live) continue;
-      const int rr = rr_red;
-      Acc s = buf[((S * W + 0) * NRT + rr) * NE];
+      const int S = it % R, pos = it / R, rr = (pos % 32) * T + pos / 32;
+      const int m = mgrp - S, row = rowS[rr];
+      if (m < p.mlo || m > lmax || row < 0) continue;
+      const Piece* const e = buf + S * Lay::step_elems + pos;
+      Acc s = Lay::get(e);
 #pragma unroll
-      for (int x = 1; x < W; ++x) acc_add(s, buf[((S * W + x) * NRT + rr) * NE]);
+      for (int x = 1; x < W; ++x) acc_add(s, Lay::get(e + x * NRT));
+      R2* const ftm = reinterpret_cast<R2*>(p.ftm) + (size_t)b * p.nrows * p.ncol;
       if constexpr (SYM) {
         // ring r gets E + O, its mirror E - O (the equator, its own mirror, E + O once)
-        Acc o = buf[((S * W + 0) * NRT + rr) * NE + 1];
+        const Piece* const eo = e + Lay::NP * Lay::piece_elems;
+        Acc o = Lay::get(eo);
 #pragma unroll
-        for (int x = 1; x < W; ++x) acc_add(o, buf[((S * W + x) * NRT + rr) * NE + 1]);
-        if (ftm_rm) {
+        for (int x = 1; x < W; ++x) acc_add(o, Lay::get(eo + x * NRT));
+        const int mirror = rowS[NRT + rr];
+        if (mirror >= 0) {
           Acc d = s;
           acc_fma(d, Real(-1), o);
-          inv2_store<DUAL>(ftm_rm, d, L, m, p.mo, half);
+          inv2_store<DUAL>(ftm + (size_t)mirror * p.ncol, d, L, m, p.mo, half);
         }
         acc_add(s, o);
       }
-      inv2_store<DUAL>(ftm_r, s, L, m, p.mo, half);
+      inv2_store<DUAL>(ftm + (size_t)row * p.ncol, s, L, m, p.mo, half);
     }
     if constexpr (Lay::NBUF == 1) __syncthreads();  // buf is rewritten by the next group
   }
   return true;
 }
 
+// CTAs per SM: two rings per lane in double keep 32 recurrences (128 registers) in flight
+template <typename Real, int T>
+constexpr int inv2_min_ctas() {
+  return sizeof(Real) == 8 && T == 2 ? 2 : 3;
+}
+
 template <typename Real, bool DUAL, int T, int W, int R, bool VST, bool SYM>
-__global__ void __launch_bounds__(W * 32, 3) lat_inv2_kernel(const Inv2Params p) {
+__global__ void __launch_bounds__(W * 32, inv2_min_ctas<Real, T>()) lat_inv2_kernel(const Inv2Params p) {
   chain_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bool live = false;
@@ -401,7 +440,7 @@ __global__ void __launch_bounds__(W * 32, 3) lat_inv2_kernel(const Inv2Params p)
 // work counter until none are left; the items of the first plans (the batch orders its plans
 // by work, largest first) go first. Stops after a bounded wait ran out.
 template <typename Real, bool DUAL, int T, int W, int R, bool VST, bool SYM>
-__global__ void __launch_bounds__(W * 32, 3) lat_inv2_persistent(const Inv2Batch w) {
+__global__ void __launch_bounds__(W * 32, inv2_min_ctas<Real, T>()) lat_inv2_persistent(const Inv2Batch w) {
   using Lay = Inv2Layout<Real, DUAL, T, W, R, VST, SYM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int item;
@@ -428,8 +467,7 @@ template <typename Real, bool DUAL, int T, int R, bool VST, bool SYM>
 static cudaError_t launch_inv2_cfg(const Inv2Params& p, cudaStream_t s) {
   using Lay = Inv2Layout<Real, DUAL, T, 4, R, VST, SYM>;
   auto kern = lat_inv2_kernel<Real, DUAL, T, 4, R, VST, SYM>;
-  cudaError_t err =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::total);
+  cudaError_t err = func_limits(kern, Lay::total);
   if (err != cudaSuccess) return err;
   dim3 grid((p.nrings + Lay::NRT - 1) / Lay::NRT, (p.NB / 2) * (p.Mst1 ? p.nseg : 1),
             p.nhalf * p.batch);
@@ -442,21 +480,28 @@ static cudaError_t launch_inv2_dual(bool dual, const Inv2Params& p, cudaStream_t
               : launch_inv2_cfg<Real, false, T, 8, VST, SYM>(p, s);
 }
 
-// tile bit 0: one ring per lane (float; double always has one); bit 1: start values read
+// tile bit 0: one ring per lane (else two, except in double on ring pairs, whose sums would
+// not fit shared memory); bit 1: start values read
 // from global memory instead of staged in shared memory. 8-step groups (the start tables'
 // alignment).
 template <bool SYM>
 static cudaError_t launch_inv2_prec(bool fp64, bool dual, const Inv2Params& p, cudaStream_t s) {
   const bool vst = (p.tile & 2) == 0;
+#define S2B_INV2(REAL)                                              \
+  if (p.tile & 1)                                                   \
+    return vst ? launch_inv2_dual<REAL, 1, true, SYM>(dual, p, s)   \
+               : launch_inv2_dual<REAL, 1, false, SYM>(dual, p, s); \
+  return vst ? launch_inv2_dual<REAL, 2, true, SYM>(dual, p, s)     \
+             : launch_inv2_dual<REAL, 2, false, SYM>(dual, p, s)
   if (!fp64) {
-    if (p.tile & 1)
-      return vst ? launch_inv2_dual<float, 1, true, SYM>(dual, p, s)
-                 : launch_inv2_dual<float, 1, false, SYM>(dual, p, s);
-    return vst ? launch_inv2_dual<float, 2, true, SYM>(dual, p, s)
-               : launch_inv2_dual<float, 2, false, SYM>(dual, p, s);
+    S2B_INV2(float);
+  }
+  if constexpr (!SYM) {
+    S2B_INV2(double);
   }
   return vst ? launch_inv2_dual<double, 1, true, SYM>(dual, p, s)
              : launch_inv2_dual<double, 1, false, SYM>(dual, p, s);
+#undef S2B_INV2
 }
 
 // CTAs of a persistent launch: what fits on the device at once, at most one per item
@@ -479,8 +524,7 @@ static cudaError_t launch_inv2_batch_cfg(const Inv2Params* ps, int n, int* count
                                          cudaStream_t s) {
   using Lay = Inv2Layout<Real, DUAL, T, 4, R, VST, SYM>;
   auto kern = lat_inv2_persistent<Real, DUAL, T, 4, R, VST, SYM>;
-  cudaError_t err =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::total);
+  cudaError_t err = func_limits(kern, Lay::total);
   if (err != cudaSuccess) return err;
   Inv2Batch w{};
   w.nplans = n;
@@ -520,6 +564,11 @@ static cudaError_t launch_inv2_batch_prec(bool fp64, bool dual, const Inv2Params
     if (vst) S2B_INV2B(float, 2, true);
     S2B_INV2B(float, 2, false);
   }
+  if constexpr (!SYM)
+    if (!one) {
+      if (vst) S2B_INV2B(double, 2, true);
+      S2B_INV2B(double, 2, false);
+    }
   if (vst) S2B_INV2B(double, 1, true);
   S2B_INV2B(double, 1, false);
 #undef S2B_INV2B

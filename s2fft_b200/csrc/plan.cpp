@@ -922,9 +922,14 @@ static int build_plan(s2b_plan* p) {
     // launch shape of the inverse kernel, measured at L = 256 ... 1024 (MW, HEALPix; float):
     // eight segments along m (against four: 10-11 % faster at L = 256 and 512 with the
     // tiles below, 1 % at 1024), start values read from global memory (shared memory for 3
-    // CTAs per SM), two rings per lane in float from L = 512 and one below
+    // CTAs per SM), two rings per lane in float from L = 512 and one below; in double two from
+    // L = 400 at spin 0 (66 us against 69, L = 1024 451 against 531), 250 otherwise (L = 200 36
+    // against 33, L = 256 38 against 45)
     p->inv_nseg = kInvSegMax;
-    p->tile_inv = (!p->fp64 && L >= 512) ? 2 : 3;
+    if (p->fp64)
+      p->tile_inv = L >= (d.spin != 0 ? 250 : 400) ? 2 : 3;
+    else
+      p->tile_inv = L >= 512 ? 2 : 3;
     // symmetric inverse: one ring pair per lane (two would double the partial sums in
     // shared memory and drop to 2 CTAs per SM; measured slower at L = 256 ... 2048)
     if (p->inv_sym) p->tile_inv = 3;
