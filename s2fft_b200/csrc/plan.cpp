@@ -929,7 +929,8 @@ static int build_plan(s2b_plan* p) {
     if (p->fp64)
       p->tile_inv = L >= (d.spin != 0 ? 250 : 400) ? 2 : 3;
     else
-      p->tile_inv = L >= 512 ? 2 : 3;
+      // (spin != 0 from L = 640 one again: GL L = 1400, spin 2: 927 us against 941)
+      p->tile_inv = L >= 512 && (d.spin == 0 || L < 640) ? 2 : 3;
     // symmetric inverse: one ring pair per lane (two would double the partial sums in
     // shared memory and drop to 2 CTAs per SM; measured slower at L = 256 ... 2048)
     if (p->inv_sym) p->tile_inv = 3;
