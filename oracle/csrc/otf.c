@@ -135,7 +135,8 @@ typedef struct {
         const double w = d0[k] * P->vsign[(size_t)wrap(col, 2 * L - 1) * n + k] * exp(lr[k]); \
         TERM(col, col + mo, k, w);                                                         \
       }                                                                                    \
-      for (int k = (lind - 1 < 0 ? 0 : lind - 1); k <= lind; ++k) {                        \
+      /* at L = 2 this column of half 0 is m = 0, which half 1 assigns after it */         \
+      for (int k = L == 2 && i == 0 ? n : lind - 1 < 0 ? 0 : lind - 1; k <= lind; ++k) {   \
         const int col = sind + sgn;                                                        \
         const double w = d1[k] * P->vsign[(size_t)wrap(col, 2 * L - 1) * n + k] * exp(lr[k]); \
         TERM(col, col + mo, k, w);                                                         \

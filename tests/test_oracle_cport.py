@@ -39,6 +39,20 @@ def test_steps_match_numpy_restatement(rng, L, spin, sampling, reality, L0, nsid
     assert relerr(d[fin], c[fin]) < 1e-13
 
 
+@pytest.mark.parametrize("sampling", ["mw", "mwss", "dh", "gl"])
+@pytest.mark.parametrize("L", [2, 3, 4])
+@pytest.mark.parametrize("spin,reality", [(0, False), (1, False), (-1, False), (0, True)])
+def test_smallest_transforms_match_numpy(rng, L, sampling, spin, reality):
+    """At L = 2 the two halves of the recursion meet in the column m = 0."""
+    shape = oracle.samples.f_shape(L, sampling)
+    f = rng.standard_normal(shape) + (0 if reality else 1j * rng.standard_normal(shape))
+    flm = oracle.signal.generate_flm(rng, L, abs(spin), spin, reality)
+    for call, x in ((oracle.spherical.forward, f), (oracle.spherical.inverse, flm)):
+        a = call(x, L, spin, None, sampling, reality=reality, backend="numpy")
+        b = call(x, L, spin, None, sampling, reality=reality, backend="c")
+        assert relerr(b, a) < 1e-13
+
+
 def test_transforms_match_golden(golden):
     data, index = golden
     n = 0
