@@ -574,7 +574,6 @@ __global__ void __launch_bounds__(kRotTab) rotate_tables_kernel(RotParams p) {
 }
 
 constexpr int kWalkThreads = 128;  // also the steps of a staged chunk
-constexpr int kWalkDead = -192;    // entries below 2^-192 do not contribute
 
 // The rotation. For fixed (l, m) the values along n obey
 //   a_n d_{m,n-1} + a_{n+1} d_{m,n+1} = 2 (n cos b - m)/sin b d_{m,n},
@@ -591,11 +590,16 @@ constexpr int kWalkDead = -192;    // entries below 2^-192 do not contribute
 // rest by the same symmetry. Half of the CTA's warps walk orders m >= 0, half the orders -m.
 // beta is folded to (0, pi/2] first (d(pi - b)_{m,n} = (-1)^{l+m} d(b)_{m,-n}), where m - n
 // and n (1 - cos b) keep t accurate.
-// Values below 2^-192 (the classically forbidden range) are carried as x 2^e and only
-// stepped; their products are left out: at most 2^-192 of a coefficient. The exponents are
-// renewed every G steps, between which a value grows by less than 2^100 (G = 4 for
-// sin(b/2) >= 2^-16, else 1). A non-finite coefficient makes its degree NaN, as a product
-// with a zero would.
+// Values below 2^dead (far in the classically forbidden range) are carried as x 2^e and only
+// stepped; their products are left out. The exponents are renewed every G steps (G = 4 for
+// sin(b/2) >= 2^-16, else 1), between which a value grows by less than 2^(G bits),
+// 2^bits > 2 sqrt(2L) cot(b/2); dead = -1021 + G bits is as low as the renewal's factors and the
+// value before the last one stay normal numbers. So entries down to 2^(dead + (G-1) bits) keep
+// their digits (L = 1024: 2^-965 for b = pi/2, 2^-937 for 0.2, 2^-909 for 0.01): a single
+// coefficient gives its column of d. (Summing from 2^-192 on only, beta = 0.2 / 0.8: L = 256
+// 43 / 38 us against 39 / 33, whose warps reach the plain loop earlier; L = 1024 620 / 589
+// against 619 / 603; L = 2048 4157 / 4042 against 4248 / 4165.)
+// A non-finite coefficient makes its degree NaN, as a product with a zero would.
 // Grid: (order tiles, degrees from the largest, maps). Bound by the FP64 pipe (six operations
 // per value) and the shared-memory broadcasts (48 bytes per step for the R orders of a lane),
 // with no reduction across lanes: L = 1024, one float64 map, 0.49-0.63 ms over beta (2.6-3.3 ms
@@ -640,7 +644,7 @@ __global__ void __launch_bounds__(kWalkThreads, 4) rotate_walk_kernel(RotParams 
       int d;
       double x = frexp(f2.m / (fa.m * fb.m) * (c.m * s.m) * ig, &d);
       const int ex = f2.e - fa.e - fb.e + c.e + s.e + d;
-      if (ex >= kWalkDead || x == 0.0)
+      if (ex >= p.dead || x == 0.0)
         x = ldexp(x, ex);
       else
         e[r] = ex;
@@ -714,11 +718,11 @@ __global__ void __launch_bounds__(kWalkThreads, 4) rotate_walk_kernel(RotParams 
     for (int r = 0; r < R; ++r) {
       if (e[r] < 0) {
         const int x = ((__double2hiint(v[r]) >> 20) & 0x7ff) - 1022, en = e[r] + x;
-        const int sh = en >= kWalkDead ? e[r] : -x;
+        const int sh = en >= p.dead ? e[r] : -x;
         const double f = __hiloint2double((1023 + sh) << 20, 0);
         v[r] *= f;
         vp[r] *= f;
-        e[r] = en >= kWalkDead ? 0 : en;
+        e[r] = en >= p.dead ? 0 : en;
       }
     }
   };
@@ -992,7 +996,9 @@ cudaError_t rotate_launch(RotParams p, cudaStream_t s) {
     rotate_planes_kernel<R2><<<(unsigned)blocks, 256, 0, s>>>(p);
     return cudaGetLastError();
   }
-  if (sn < 0x1p-16L) return launch_walk<R2, 2, 1>(p, s);
+  const int G = sn < 0x1p-16L ? 1 : 4;
+  p.dead = -1021 + G * (int)ceill(log2l(2.0L * sqrtl(2.0L * L) * c / sn));
+  if (G == 1) return launch_walk<R2, 2, 1>(p, s);
   // two orders per lane leave enough warps up to here (L = 1024, beta = 0.2 / 1.5: 626 / 485 us
   // against 664 / 473 with four; L = 1500: 1784 / 1412 against 1803 / 1340), four need fewer
   // broadcasts per order beyond (L = 2048: 4155 / 3222 us against 4282 / 3463)

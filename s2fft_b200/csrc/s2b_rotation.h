@@ -35,6 +35,7 @@ struct RotParams {
   int flip;             // beta stands for pi - b
   int par;              // d of beta has the further sign (-1)^{m-n}
   int nan;              // beta is not finite
+  int dead;             // the walk's values below 2^dead are not summed
   // workspace (rotate_bind_workspace):
   double2* ea;     // exp(-i m alpha), m in [-(L-1), L-1]
   double2* eg;     // exp(-i n gamma)
