@@ -146,7 +146,7 @@ __device__ __forceinline__ void chain_enter() {
 cudaError_t func_limits_of(const void* kernel, int smem, int carveout);  // stages.cu
 
 // Dynamic shared memory limit (at least smem bytes) and, unless carveout < 0, shared-memory
-// carveout of a kernel on the current device: set when they change instead of before every
+// carveout of a kernel in the current context: set when they change instead of before every
 // launch. The limit is only raised, so that a launch from another thread keeps its own.
 template <typename... KArgs>
 inline cudaError_t func_limits(void (*kernel)(KArgs...), size_t smem, int carveout = -1) {

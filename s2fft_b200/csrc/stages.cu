@@ -5,6 +5,7 @@
 //  * inverse pole rows in closed form (spherical.py:175-184);
 //  * forward epilogue: projected sums -> flm (g_{l,m}, pole terms, normalisation,
 //    reality mirror, spin/L_lower mask, (-1)^s; spherical.py:566-588).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -519,18 +520,49 @@ cudaError_t launch_sub(bool fp64, long n, const void* x, const void* y, void* z,
   return cudaGetLastError();
 }
 
-// What the current process has set, per kernel and device (one entry per kernel instance).
+// The driver's id of the calling thread's context, unique for the life of the program; 0 where it
+// cannot be told.
+static unsigned long long context_id() {
+  using Current = CUresult(CUDAAPI*)(CUcontext*);
+  using Id = CUresult(CUDAAPI*)(CUcontext, unsigned long long*);
+  struct Entry {
+    Current current = nullptr;
+    Id id = nullptr;
+    Entry() {
+      void *a = nullptr, *b = nullptr;
+      cudaDriverEntryPointQueryResult ra, rb;
+      if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &a, 12000, cudaEnableDefault, &ra) ==
+              cudaSuccess &&
+          cudaGetDriverEntryPointByVersion("cuCtxGetId", &b, 12000, cudaEnableDefault, &rb) ==
+              cudaSuccess &&
+          ra == cudaDriverEntryPointSuccess && rb == cudaDriverEntryPointSuccess) {
+        current = reinterpret_cast<Current>(a);
+        id = reinterpret_cast<Id>(b);
+      }
+    }
+  };
+  static const Entry entry;
+  CUcontext c = nullptr;
+  unsigned long long id = 0;
+  if (!entry.id || entry.current(&c) != CUDA_SUCCESS || !c || entry.id(c, &id) != CUDA_SUCCESS)
+    return 0;
+  return id;
+}
+
+// A kernel's limits live in a context: what has been set is kept per context (an id is not given
+// out twice, so a reset device or a further context begins anew), and set every time where the
+// context cannot be told.
 cudaError_t func_limits_of(const void* kernel, int smem, int carveout) {
   struct Limits {
     int smem = 0, carveout = -1;
   };
   static std::mutex mu;
-  static std::map<std::pair<const void*, int>, Limits> set;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
+  static std::map<std::pair<const void*, unsigned long long>, Limits> set;
+  const unsigned long long ctx = context_id();
+  cudaError_t e;
   std::lock_guard<std::mutex> lk(mu);
-  Limits& l = set[{kernel, dev}];
+  Limits once;
+  Limits& l = ctx ? set[{kernel, ctx}] : once;
   if (smem > l.smem) {
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
