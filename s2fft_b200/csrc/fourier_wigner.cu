@@ -27,7 +27,7 @@
 //
 // Frequencies are stored "value mod length", which is what upstream's fftshift /
 // ifftshift pairs amount to. One CTA transforms a row or column, on the register engine
-// (s2b_fft_reg.h) where its working lengths reach, else (and in the adjoints and the gamma
+// (s2b_fft_reg.h) where that is faster (fw_reg_from), else (and in the adjoints and the gamma
 // DFT) by the shared-memory passes of s2b_fft_dev.h.
 #include <cuda_runtime.h>
 
@@ -1146,13 +1146,53 @@ cudaError_t launch_fft(K kernel, dim3 grid, int M, size_t smem, cudaStream_t st,
 
 enum FwChain { kFwRowsInv, kFwRowsFwd, kFwColsInv, kFwColsFwd };
 
+// log2 of the least working length at which a chain runs on the register engine; blu: nphi is
+// Bluestein's (the columns forward run on Q points, nphi as Bluestein's in any case). Below, its
+// M / 16 threads are too few (N = 8, MW unless a power of two is meant, us, passes -> engine):
+//   rows inverse    float L = 64 6.3 -> 7.7, 128 11.9 -> 13.5, 129 23.1 -> 16.8; double 64 7.3 -> 9.4,
+//                   96 13.0 -> 13.6, 128 19.8 -> 17.3, 129 30.7 -> 24.4; powers of two (MWSS): float
+//                   L = 128 7.3 -> 5.6, double 128 7.8 -> 8.0, 256 25.3 -> 16.2
+//   rows forward    float L = 64 6.5 -> 6.1, 128 12.3 -> 11.9; double 64 7.4 -> 7.5, 65 10.6 -> 9.4;
+//                   powers of two: float L = 128 7.2 -> 5.3, double 128 7.9 -> 8.3, 256 23.5 -> 16.3
+//   columns inverse float L = 128 21.6 -> 28.2, 129 42.2 -> 31.3; double 96 23.7 -> 24.6, 129 56.0 ->
+//                   43.7; powers of two: float L = 256 34.1 -> 49.8, 512 (N = 3) 55.0 -> 43.8
+//   columns forward float L = 128 40.8 -> 43.1, 129 90.9 -> 72.9; double 64 19.5 -> 25.9, 65 38.7 ->
+//                   29.6; powers of two: float L = 256 127 -> 145, 512 (N = 3) 214 -> 191
+// L = 128 in all, inverse + forward: float 231 us, 242 with the engine from 256 points on.
+template <typename Real>
+constexpr int fw_reg_from(FwChain c, bool blu) {
+  constexpr bool f32 = sizeof(Real) == 4;
+  switch (c) {
+    case kFwRowsInv: return blu ? 10 : f32 ? 8 : 9;
+    case kFwRowsFwd: return blu || f32 ? 8 : 9;
+    case kFwColsInv: return 10;
+    default: return !blu ? 11 : f32 ? 10 : 9;
+  }
+}
+
+// the kernel of chain C on 2^LOGM points (nullptr where the rule never takes it)
+template <typename Real, int LOGM, FwChain C>
+constexpr auto fw_reg_kernel() -> void (*)(FWFftParams<Real>) {
+  if constexpr (LOGM < fw_reg_from<Real>(C, true) && LOGM < fw_reg_from<Real>(C, false))
+    return nullptr;
+  else if constexpr (C == kFwRowsInv)
+    return fw_rows_inv_reg_kernel<Real, LOGM>;
+  else if constexpr (C == kFwRowsFwd)
+    return fw_rows_fwd_reg_kernel<Real, LOGM>;
+  else if constexpr (C == kFwColsInv)
+    return fw_cols_inv_reg_kernel<Real, LOGM>;
+  else
+    return fw_cols_fwd_reg_kernel<Real, LOGM>;
+}
+
 template <typename Real, int LOGM>
 cudaError_t launch_reg(FwChain c, dim3 grid, int extra, cudaStream_t st,
                        const FWFftParams<Real>& f) {
-  void (*k)(FWFftParams<Real>) = c == kFwRowsInv   ? fw_rows_inv_reg_kernel<Real, LOGM>
-                                 : c == kFwRowsFwd ? fw_rows_fwd_reg_kernel<Real, LOGM>
-                                 : c == kFwColsInv ? fw_cols_inv_reg_kernel<Real, LOGM>
-                                                   : fw_cols_fwd_reg_kernel<Real, LOGM>;
+  if (LOGM < fw_reg_from<Real>(c, f.dphi.bluestein != 0)) return cudaErrorNotSupported;
+  void (*k)(FWFftParams<Real>) = c == kFwRowsInv   ? fw_reg_kernel<Real, LOGM, kFwRowsInv>()
+                                 : c == kFwRowsFwd ? fw_reg_kernel<Real, LOGM, kFwRowsFwd>()
+                                 : c == kFwColsInv ? fw_reg_kernel<Real, LOGM, kFwColsInv>()
+                                                   : fw_reg_kernel<Real, LOGM, kFwColsFwd>();
   const size_t smem =
       ((size_t)RegFFT<LOGM, 1>::SMEM_ELEMS + extra) * sizeof(typename C2<Real>::t);
   // shared memory for the CTAs of the launch bounds, the rest L1 for the tables
@@ -1164,7 +1204,8 @@ cudaError_t launch_reg(FwChain c, dim3 grid, int extra, cudaStream_t st,
   return cudaGetLastError();
 }
 
-// A chain on the register engine with working length M; cudaErrorNotSupported where it has none.
+// A chain on the register engine with working length M; cudaErrorNotSupported where the rule
+// leaves it to the shared-memory passes.
 template <typename Real>
 cudaError_t launch_chain(FwChain c, dim3 grid, int M, int extra, cudaStream_t st,
                          const FWFftParams<Real>& f) {
@@ -1222,14 +1263,11 @@ template <typename Real>
 int inverse_chain(const s2b_fw_plan* p, int E, const FWSlices& sl, const double* delta,
                   const void* coef, void* maps, int nmajor, int groups, char* ws,
                   const FWLayout& lay, cudaStream_t st) {
-  using R2 = typename C2<Real>::t;
   void* A = ws;
   void* B = ws + lay.a;
   int rc = contract<Real>(p, false, E, sl, delta, coef, A, st);
   if (rc) return rc;
   FWFftParams<Real> f = fft_params<Real>(p, E, sl);
-  const int M = f.dphi.M;
-  const size_t smem = (size_t)padded_len(M) * sizeof(R2);
   f.in = A;
   f.out = B;
   FW_CK(launch_dft<Real>(kFwColsInv, dim3(2 * p->L - 1, E), st, f));
@@ -1259,7 +1297,6 @@ int forward_chain(const s2b_fw_plan* p, int E, const FWSlices& sl, const double*
   FWFftParams<Real> f = fft_params<Real>(p, E, sl);
   f.quads = qQ;
   f.wconv = wk;
-  const int M = f.dphi.M;
   f.in = maps;
   f.out = B;
   f.nmajor = nmajor;

@@ -1,6 +1,6 @@
-"""The Fourier-Wigner FFT chains where their working lengths change: the shared-memory passes
-below 256 points, the register engine from there on, power-of-two rings (mwss) beside
-Bluestein's, on random SO(3) samples, so that every sampled value counts."""
+"""The Fourier-Wigner FFT chains where their working lengths and routes change: the shared-memory
+passes and, per chain and precision from 256 to 2048 points on, the register engine, power-of-two
+rings (mwss) beside Bluestein's, on random SO(3) samples, so that every sampled value counts."""
 
 import numpy as np
 import pytest
@@ -37,8 +37,8 @@ def test_against_oracle(s2b, rng, sampling, L):
         assert relerr(fw.forward_transform(f, L, N, **kw), gref) < tol
 
 
-@pytest.mark.parametrize("sampling", ["mw", "mwss"])
-@pytest.mark.parametrize("L", [128, 129, 256])
+@pytest.mark.parametrize("sampling,L", [(s, L) for s in ("mw", "mwss") for L in (128, 129, 256)]
+                         + [("mwss", 512)])
 def test_against_the_recursion(s2b, rng, sampling, L):
     """Larger lengths against the recursion-based transforms of the same library."""
     N = 2
@@ -46,3 +46,6 @@ def test_against_the_recursion(s2b, rng, sampling, L):
     f = s2b.fourier_wigner.inverse_transform(flmn, L, N, sampling=sampling)
     assert relerr(f, s2b.wigner.inverse(flmn, L, N, sampling=sampling)) < 1e-10
     assert relerr(s2b.fourier_wigner.forward_transform(f, L, N, sampling=sampling), flmn) < 1e-10
+    kw = dict(sampling=sampling, precision="f32")
+    assert relerr(s2b.fourier_wigner.inverse_transform(flmn, L, N, **kw), f) < 1e-5
+    assert relerr(s2b.fourier_wigner.forward_transform(f, L, N, **kw), flmn) < 1e-5
