@@ -443,6 +443,7 @@ struct s2b_plan {
   // (col_f1, col_f2), else they are col_d1, col_d2 and Mreg = 0
   int col_f1 = 0, col_f2 = 0, Mreg = 0;
   bool col_pruned = false;
+  bool col_table_tw = false;  // Mreg = 0: every twiddle of the passes from the table
   void* col_ph = nullptr;  // column chain: chirp * half-sample phase / n1 per 4L-bin
   // start tables of the inverse rings (inverse and its adjoint), ring -> column map of the
   // adjoint spectra (recursed rings first, then north / south pole), adjoint chain table
@@ -999,8 +1000,8 @@ static int build_plan(s2b_plan* p) {
     p->col_d2 = fb.add(4 * L);
     p->M1 = fb.descs[p->col_d1].M;
     p->M2 = fb.descs[p->col_d2].M;
-    // Register engine: one working length for both transforms. When 4L is a power of two, 4L
-    // (a theta length of 2L points then runs as Bluestein's, too). Else Bluestein's for both:
+    // Register engine: one working length for both transforms. When 4L is a power of two, 4L.
+    // Else Bluestein's for both:
     // the 4L-point transform has 2L inputs, so 6L - 1 points hold its convolution (8L - 1
     // without that: half as many band-limits would need twice the length).
     const int n1 = fb.descs[p->col_d1].n, n2 = 4 * L, top = p->fp64 ? 4096 : 8192;
@@ -1013,9 +1014,13 @@ static int build_plan(s2b_plan* p) {
     // a theta length that is a power of two needs no Bluestein in the shared-memory passes.
     if (L >= 192 && Mr <= top && (n1 & (n1 - 1)) != 0) {
       p->Mreg = Mr;
-      if (p->M1 != Mr || !fb.descs[p->col_d1].bluestein) p->col_f1 = fb.add_bluestein(n1, Mr, n1);
+      if (p->M1 != Mr) p->col_f1 = fb.add_bluestein(n1, Mr, n1);
       if (p->col_pruned) p->col_f2 = fb.add_bluestein(n2, Mr, 2 * L);
     }
+    // MW with L a power of two: the passes with the engine's twiddles, whose error they would
+    // exceed otherwise (float, L = 64 and 128: 4.1e-7 and 4.2e-7 against 3.5e-7 and 3.7e-7, with
+    // them 3.3e-7 and 3.6e-7; time 30 and 41 us, on the engine 48 at L = 128)
+    p->col_table_tw = !p->Mreg && p->fwd_mode == 1 && !p->col_pruned && L < 192;
   }
   p->maxM = 2;
   if (d.sampling == S2B_HEALPIX) {
@@ -1672,6 +1677,7 @@ static int fwd_stage_pre(s2b_plan* p, const void* f, char* ws, cudaStream_t s, F
     cp.d1 = p->descs + p->col_f1;
     cp.d2 = p->descs + p->col_f2;
     cp.Mreg = p->Mreg;
+    cp.table_tw = p->col_table_tw;
     cp.pruned = p->col_pruned;
     cp.ph = p->col_ph;
     cp.pole = p->col_pole;
@@ -1970,6 +1976,7 @@ static int run_pre_forward(s2b_plan* p, const void* K, const void* f, void* flm,
     cp.d1 = p->descs + p->col_f1;
     cp.d2 = p->descs + p->col_f2;
     cp.Mreg = p->Mreg;
+    cp.table_tw = p->col_table_tw;
     cp.pruned = p->col_pruned;
     cp.ph = p->col_ph;
     cp.pole = p->col_pole;

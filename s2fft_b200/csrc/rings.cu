@@ -466,8 +466,9 @@ __device__ __forceinline__ void cols_emit(const ColsParams<Real>& p, int b, int 
     });
 }
 
-// The shared-memory passes, for working lengths beyond the register engine's.
-template <typename Real>
+// The shared-memory passes: band-limits below 192, MWSS with L a power of two and working lengths
+// beyond the register engine's (the plan's rule). TW: see fft_pass.
+template <typename Real, bool TW>
 __global__ void __launch_bounds__(512, reg_min_blocks<Real>(0)) mw_cols_kernel(ColsParams<Real> p) {
   chain_enter();
   using R2 = typename C2<Real>::t;
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(512, reg_min_blocks<Real>(0)) mw_cols_kernel(C
   const int phi = L - 1;
   const int n2 = d2.n;  // 4L
   const R2* __restrict__ ph = reinterpret_cast<const R2*>(p.ph);
-  dft_run<Real>(s1, d1, p.tb, false, load1);
+  dft_run<Real, TW>(s1, d1, p.tb, false, load1);
   for (int pp = plo + (int)threadIdx.x; pp <= phi; pp += blockDim.x) {
     const int j = pmod(pp, n1);
     const R2 g = d1.bluestein ? s1[pidx(j)] : s1[pidx(bitrev(j, d1.logM))];
@@ -519,7 +520,7 @@ __global__ void __launch_bounds__(512, reg_min_blocks<Real>(0)) mw_cols_kernel(C
   const R2* __restrict__ pole = (p.mw && par) ? reinterpret_cast<const R2*>(p.pole) : nullptr;
   const R2 xpole = pole ? c[L - 1] : czero<R2>();
   const R2 nyq = (!p.mw && p.nyq_split) ? tmp[0] : czero<R2>();
-  dft_run<Real>(s2, d2, p.tb, true, load2);
+  dft_run<Real, TW>(s2, d2, p.tb, true, load2);
   auto chain = [&](int t) -> R2 {
     R2 u = dft_get<Real>(s2, d2, p.tb, true, t);
     if (pole) u = cadd(u, cmul(xpole, pole[t]));
@@ -880,8 +881,8 @@ cudaError_t launch_mw_cols(const ColsParams<Real>& p, int ncm, int batch, int M1
   }
   // one DFT buffer plus the 2L bins carried between the two transforms
   const size_t smem = (size_t)(padded_len(M1 > M2 ? M1 : M2) + 2 * p.L) * sizeof(R2);
-  return launch_fft_kernel<Real>(mw_cols_kernel<Real>, grid, fft_threads(M1 > M2 ? M1 : M2),
-                                 smem, p, s);
+  return launch_fft_kernel<Real>(p.table_tw ? mw_cols_kernel<Real, true> : mw_cols_kernel<Real, false>,
+                                 grid, fft_threads(M1 > M2 ? M1 : M2), smem, p, s);
 }
 
 template <typename Real>

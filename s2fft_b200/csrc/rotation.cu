@@ -595,7 +595,7 @@ constexpr int kWalkThreads = 128;  // also the steps of a staged chunk
 // sin(b/2) >= 2^-16, else 1), between which a value grows by less than 2^(G bits),
 // 2^bits > 2 sqrt(2L) cot(b/2); dead = -1021 + G bits is as low as the renewal's factors and the
 // value before the last one stay normal numbers. So entries down to 2^(dead + (G-1) bits) keep
-// their digits (L = 1024: 2^-965 for b = pi/2, 2^-937 for 0.2, 2^-909 for 0.01): a single
+// their digits (L = 1024: 2^-972 for b = pi/2, 2^-951 for 0.2, 2^-916 for 0.01): a single
 // coefficient gives its column of d. (Summing from 2^-192 on only, beta = 0.2 / 0.8: L = 256
 // 43 / 38 us against 39 / 33, whose warps reach the plain loop earlier; L = 1024 620 / 589
 // against 619 / 603; L = 2048 4157 / 4042 against 4248 / 4165.)

@@ -81,6 +81,7 @@ struct ColsParams {
   const FFTDesc* d2;    // inverse DFT of length 4L
   int Mreg;             // working length of d1 and d2 on the register engine (0: not used)
   int pruned;           // register engine, d2: Bluestein's of the 2L bins from p = -L on
+  int table_tw;         // shared-memory passes with every twiddle from the table
   const double* weights;// 2L+1 MWSS(2L) transform weights
   const void* ph;       // [4L] complex factor of theta-DFT bin p (at p mod 4L), 0 outside
   const void* ph_adj;   // [4L] adjoint chain: conj(half-sample phase) / n1 (at p mod 4L)
