@@ -1562,6 +1562,13 @@ static int run_forward_adjoint(s2b_plan* p, const void* gflm, void* gf, char* ws
   lp.mo = 0;
   lp.status = p->status;
   lp.mlo = lowm_orders(p);
+  // One ring per lane, start values staged: without segments along m there are few CTAs, and two
+  // rings per lane halve them (and staged in double leave one CTA per SM): MW, us, two rings and
+  // staged -> this: double L = 64 / 256 / 1024 spin 0 64 / 156 / 1466 -> 51 / 126 / 1311, spin 2
+  // 60 / 145 / 1891 -> 53 / 129 / 1650; float spin 0 53 / 125 / 830 -> 43 / 94 / 760, spin 2
+  // 53 / 151 -> 47 / 111. Float with spin from L = 624 on: start values from global memory (L = 608
+  // staged 460 against 468, 640 501 against 484, 1024 933 against 899).
+  lp.tile = !p->fp64 && d.spin != 0 && L >= 624 ? 3 : 1;
   S2B_CK(launch_inv2(p->fp64, p->dual, lp, s));
   if (int rc_ = run_lowm_synth(p, lp, p->fwd_rings, s)) return rc_;
   ColsParams<Real> cp{};

@@ -103,7 +103,8 @@ struct Inv2Params {
   const int* ring_row;
   int nrows, ncol, mo;
   int* status;
-  int tile;                 // 0: default rings per lane, 1: one ring per lane (more CTAs)
+  int tile;                 // bit 0: one ring per lane instead of two (more CTAs); bit 1: start
+                            // values read from global memory instead of staged
   int mlo;                  // orders m < mlo are left to the degree recursion (lowm.cu)
 };
 cudaError_t launch_inv2(bool fp64, bool dual, const Inv2Params& p, cudaStream_t s);

@@ -90,6 +90,34 @@ def test_adjoint_dot_products_high_spin(s2b, rng, sampling, spin):
     assert abs(lhs - rhs) <= 1e-10 * abs(lhs), (lhs, rhs)
 
 
+@pytest.mark.parametrize("precision,L", [("f64", 200), ("f64", 401), ("f32", 200), ("f32", 623),
+                                         ("f32", 624)])
+@pytest.mark.parametrize("sampling", ["mw", "mwss"])
+@pytest.mark.parametrize("spin", [0, 2])
+def test_forward_adjoint_launch_shapes(s2b, rng, sampling, spin, precision, L):
+    """The adjoint of the forward at band-limits of several tiles and on both sides of its choice
+    of launch shape: <A x, y> = <x, A^H y>, relative to the norms (each side's terms carry the
+    transform's relative error, 1e-10 or 1e-5)."""
+    import torch
+
+    cdt = torch.complex128 if precision == "f64" else torch.complex64
+    shape = s2b.f_shape(L, sampling)
+    fin = torch.tensor(rng.normal(size=shape) + 1j * rng.normal(size=shape), dtype=cdt,
+                       device="cuda", requires_grad=True)
+    h = torch.tensor(oracle.signal.generate_flm(rng, L, 0, spin), dtype=cdt, device="cuda")
+    flm = s2b.forward(fin, L, spin, None, sampling, precision=precision)
+    (gf,) = torch.autograd.grad(flm, fin, grad_outputs=h)
+    lhs, rhs = _vdot(flm.detach(), h), _vdot(fin.detach(), gf)
+    scale = float(flm.detach().norm() * h.norm())
+    assert abs(lhs - rhs) <= TOL[precision] * scale, (lhs, rhs, scale)
+    # every entry, against the double adjoint
+    if precision == "f32":
+        f64 = fin.detach().to(torch.complex128).requires_grad_(True)
+        (g64,) = torch.autograd.grad(s2b.forward(f64, L, spin, None, sampling), f64,
+                                     grad_outputs=h.to(torch.complex128))
+        assert relerr(gf.cpu().numpy(), g64.cpu().numpy()) < 1e-5
+
+
 def _fd_check(loss_fn, x, grad, coords, tol):
     """Central differences on the real and imaginary part of each coordinate."""
     import torch
