@@ -2401,6 +2401,20 @@ static void drop_aux(s2b_plan* p) {
   p->aux_fork = p->aux_join = nullptr;
 }
 
+// Whether the low orders of a slice run on a stream of their own (four event calls per slice and
+// direction) or follow in the slice's stream. Beside, where few slices leave room on the device, or
+// a few of the eight streams carry a second slice; MW, float, inverse / forward, us, following ->
+// beside: L = 256 N = 2 (3 slices) 86 / 149 -> 73 / 135, N = 5 (9) 206 / 374 -> 184 / 329, N = 6 (11)
+// 237 / 395 -> 225 / 419 (GL 232 / 256 -> 222 / 263, double 304 / 559 -> 284 / 558); following
+// otherwise, N = 4 (7) 153 / 292 -> 141 / 231, N = 8 (15) 314 / 557 -> 308 / 468. Below L = 128 (160
+// with four slices or more, 256 with eleven) the calls outweigh it: L = 128 N = 3 reality 69 / 82
+// beside, 64 / 91 following, N = 5 (9) 126 / 175 and 111 / 177; GL L = 160 N = 6 (11) 148 / 182 and
+// 134 / 166.
+static bool wigner_lowm_beside(int nsub, int L) {
+  return (nsub <= 5 || (nsub > s2b_plan::kMaxWStreams && nsub <= s2b_plan::kMaxWStreams + 3)) &&
+         L >= (nsub <= 3 ? 128 : nsub <= 9 ? 160 : 256);
+}
+
 static int build_wigner(s2b_plan* p) {
   const s2b_desc& d = p->d;
   p->fp64 = d.precision == S2B_F64;
@@ -2408,7 +2422,7 @@ static int build_wigner(s2b_plan* p) {
   p->nth = ntheta(d.L, d.sampling, d.nside);
   p->nphi = d.sampling == S2B_HEALPIX ? 0 : nphi_equiang(d.L, d.sampling);
   p->npix = d.sampling == S2B_HEALPIX ? 12L * d.nside * d.nside : (long)p->nth * p->nphi;
-  const int n0 = d.reality ? 0 : -(d.N - 1);
+  const int n0 = d.reality ? 0 : -(d.N - 1), nsub = d.N - n0;
   for (int n = n0; n < d.N; ++n) {
     s2b_desc sd = d;
     sd.spin = -n;
@@ -2419,9 +2433,7 @@ static int build_wigner(s2b_plan* p) {
     int rc = s2b_plan_create(&sd, &sub);
     if (rc) return rc;
     p->subs.push_back(sub);
-    // the slices run side by side already: their low orders follow in the same stream instead
-    // of on a stream of their own (four event calls per slice and direction)
-    drop_aux(sub);
+    if (!wigner_lowm_beside(nsub, d.L)) drop_aux(sub);
     // the slice n = 0 of a real signal is a real map: upstream transforms it as one
     // (wigner.py:521-530), so its MW / MWSS column chain takes the real-map corrections
     if (d.reality && n == 0 && (rc = use_real_map_chain(sub))) return rc;
