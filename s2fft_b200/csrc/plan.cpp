@@ -930,8 +930,11 @@ static int build_plan(s2b_plan* p) {
     if (p->fp64)
       p->tile_inv = L >= (d.spin != 0 ? 250 : 400) ? 2 : 3;
     else
-      // (spin != 0 from L = 640 one again: GL L = 1400, spin 2: 927 us against 941)
-      p->tile_inv = L >= 512 && (d.spin == 0 || L < 640) ? 2 : 3;
+      // (spin != 0: one again from L = 640, with about two rings per degree, DH and HEALPix, from
+      // 1024; spin 2, us, two -> one ring per lane: GL L = 640 147.5 -> 146.4, 800 235.2 -> 232.0, 1400
+      // 941 -> 925; DH 640 243.2 -> 246.5, 800 391.4 -> 393.5, 1024 702.0 -> 698.0, 1400 1733 -> 1724)
+      p->tile_inv =
+          L >= 512 && (d.spin == 0 || L < (p->inv_nrings > L + 1 ? 1024 : 640)) ? 2 : 3;
     // symmetric inverse: one ring pair per lane (two would double the partial sums in
     // shared memory and drop to 2 CTAs per SM; measured slower at L = 256 ... 2048)
     if (p->inv_sym) p->tile_inv = 3;
