@@ -118,6 +118,33 @@ def test_forward_adjoint_launch_shapes(s2b, rng, sampling, spin, precision, L):
         assert relerr(gf.cpu().numpy(), g64.cpu().numpy()) < 1e-5
 
 
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("sampling,L,nside,spin", [
+    ("mwss", 200, None, 0), ("mwss", 200, None, -2), ("gl", 257, None, 0), ("gl", 257, None, 3),
+    ("mw", 130, None, 1), ("dh", 160, None, 2), ("healpix", 130, 64, 0)])
+def test_inverse_adjoint_segments(s2b, rng, sampling, L, nside, spin, precision):
+    """The adjoint of the inverse where its rings' m-range splits into segments: <A x, y> =
+    <x, A^H y> relative to the norms, and in float every entry against the double adjoint."""
+    import torch
+
+    cdt = torch.complex128 if precision == "f64" else torch.complex64
+    shape = s2b.f_shape(L, sampling, nside)
+    x = torch.tensor(oracle.signal.generate_flm(rng, L, 0, spin), dtype=cdt, device="cuda",
+                     requires_grad=True)
+    y = torch.tensor(rng.normal(size=shape) + 1j * rng.normal(size=shape), dtype=cdt,
+                     device="cuda")
+    f = s2b.inverse(x, L, spin, nside, sampling, precision=precision)
+    (gx,) = torch.autograd.grad(f, x, grad_outputs=y)
+    lhs, rhs = _vdot(f.detach(), y), _vdot(x.detach(), gx)
+    scale = float(f.detach().norm() * y.norm())
+    assert abs(lhs - rhs) <= TOL[precision] * scale, (lhs, rhs, scale)
+    if precision == "f32":
+        x64 = x.detach().to(torch.complex128).requires_grad_(True)
+        (g64,) = torch.autograd.grad(s2b.inverse(x64, L, spin, nside, sampling), x64,
+                                     grad_outputs=y.to(torch.complex128))
+        assert relerr(gx.cpu().numpy(), g64.cpu().numpy()) < 1e-5
+
+
 def _fd_check(loss_fn, x, grad, coords, tol):
     """Central differences on the real and imaginary part of each coordinate."""
     import torch

@@ -61,3 +61,41 @@ def test_short_power_of_two_error(s2b, L):
         y = s2b.forward(f, L, precision="f32")
         e.append(np.linalg.norm(y - ref) / np.linalg.norm(ref))
     assert np.mean(e) < 3.85e-7, e
+
+
+@pytest.mark.parametrize("sampling", ["mw", "mwss"])
+@pytest.mark.parametrize("L", [341, 342, 682, 683])
+@pytest.mark.parametrize("spin,reality", [(0, True), (1, False)])
+def test_noise_at_the_length_limits(s2b, rng, sampling, L, spin, reality):
+    """White noise at the working lengths' limits (6L - 1 against 2048 and 4096, in double 4096 the
+    last): odd columns' own samples and the Nyquist bin count here, a round trip sees neither."""
+    shape = s2b.spherical.f_shape(L, sampling)
+    f = rng.standard_normal(shape) + (0 if reality else 1j * rng.standard_normal(shape))
+    ref = oracle.spherical.forward(f, L, spin, None, sampling, reality=reality, backend="c")
+    for precision, tol in (("f64", 1e-10), ("f32", 1e-5)):
+        y = s2b.forward(f, L, spin, None, sampling, reality=reality, precision=precision)
+        assert relerr(y, ref) < tol, (precision, relerr(y, ref))
+
+
+@pytest.mark.parametrize("sampling,L", [("mw", 1365), ("mwss", 1366)])
+def test_noise_at_the_longest_length(s2b, rng, sampling, L):
+    """Float: 6L - 1 = 8189 on the engine's 8192 points, and the first band-limit beyond it."""
+    shape = s2b.spherical.f_shape(L, sampling)
+    f = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    ref = oracle.spherical.forward(f, L, 1, None, sampling, backend="c")
+    y = s2b.forward(f, L, 1, None, sampling, precision="f32")
+    assert relerr(y, ref) < 1e-5, relerr(y, ref)
+
+
+@pytest.mark.parametrize("sampling", ["mw", "mwss"])
+@pytest.mark.parametrize("L", [150, 192, 200, 256])
+@pytest.mark.parametrize("spin,reality", [(0, False), (0, True), (-2, False)])
+def test_precompute_forward_against_on_the_fly(s2b, rng, sampling, L, spin, reality):
+    """The chain's raw layout (precompute forward) on both routes, on white noise: the same map by
+    the on-the-fly transform, whose chain the tests above hold to the oracle."""
+    shape = s2b.spherical.f_shape(L, sampling)
+    f = rng.standard_normal(shape) + (0 if reality else 1j * rng.standard_normal(shape))
+    ref = s2b.forward(f, L, spin, None, sampling, reality=reality)
+    for precision, tol in (("f64", 1e-10), ("f32", 1e-5)):
+        y = s2b.precompute.forward(f, L, spin, None, sampling, reality, precision=precision)
+        assert relerr(y, ref) < tol, (precision, relerr(y, ref))

@@ -447,6 +447,25 @@ def test_bf16x3_tensor_core_healpix(s2b, rng, reality):
     assert relerr(g, g64) < 5e-5
 
 
+@pytest.mark.parametrize("sampling,L,nside,spin,reality", [
+    ("healpix", 128, 64, 0, False), ("healpix", 130, 64, 0, True), ("mw", 200, None, 2, False),
+    ("mwss", 129, None, -1, False), ("dh", 150, None, 0, True)])
+def test_bf16x3_skipped_blocks(s2b, rng, sampling, L, nside, spin, reality):
+    """Several row tiles and chunks, so that blocks of zeros are left out, in the doubled K dimension
+    of HEALPix too, in both directions, with maps in two groups and an order axis that is no multiple
+    of a CTA's columns: against the double precompute path."""
+    B = 66
+    shape = s2b.f_shape(L, sampling, nside)
+    flms = np.stack([oracle.signal.generate_flm(rng, L, 0, spin, reality) for _ in range(B)])
+    f = rng.standard_normal((B,) + shape) + (0 if reality else 1j * rng.standard_normal((B,) + shape))
+    for call, x, forward in ((s2b.precompute.inverse, flms, False), (s2b.precompute.forward, f, True)):
+        K = s2b.precompute.spin_spherical_kernel(L, spin, reality, sampling, nside, forward,
+                                                 precision="bf16x3")
+        y = call(x, L, spin, K, sampling, reality, nside=nside, precision="bf16x3")
+        ref = call(x, L, spin, None, sampling, reality, nside=nside)
+        assert relerr(y, ref) < 5e-5, (forward, relerr(y, ref))
+
+
 @pytest.mark.parametrize("sampling", ["mw", "mwss", "dh", "gl"])
 @pytest.mark.parametrize("spin,reality", [(0, False), (-2, False), (1, False), (0, True),
                                           (2, True)])
