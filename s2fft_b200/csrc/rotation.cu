@@ -973,7 +973,10 @@ cudaError_t rotate_launch(RotParams p, cudaStream_t s) {
   sn = fabsl(sn);
   p.flip = c < sn;
   if (p.flip) std::swap(c, sn);
-  sn = fmaxl(sn, ldexpl(1.0L, -101));  // below, the rotation is the identity to rounding
+  // below 2^-500 (the factors 2^bits of a step would leave the double range) the rotation is the
+  // identity: its values run on 2^-500 and all that is not near 1 is left out
+  const bool ident = sn < ldexpl(1.0L, -500);
+  if (ident) sn = ldexpl(1.0L, -500);
   p.ch = (double)c;
   p.cl = (double)(c - p.ch);
   p.sh = (double)sn;
@@ -997,7 +1000,7 @@ cudaError_t rotate_launch(RotParams p, cudaStream_t s) {
     return cudaGetLastError();
   }
   const int G = sn < 0x1p-16L ? 1 : 4;
-  p.dead = -1021 + G * (int)ceill(log2l(2.0L * sqrtl(2.0L * L) * c / sn));
+  p.dead = ident ? -400 : -1021 + G * (int)ceill(log2l(2.0L * sqrtl(2.0L * L) * c / sn));
   if (G == 1) return launch_walk<R2, 2, 1>(p, s);
   // two orders per lane leave enough warps up to here (L = 1024, beta = 0.2 / 1.5: 626 / 485 us
   // against 664 / 473 with four; L = 1500: 1784 / 1412 against 1803 / 1340), four need fewer

@@ -68,3 +68,33 @@ def test_tiny_entries_keep_their_digits(s2b, L, beta):
         assert (err[normal] <= 1e-15 * L * scale[normal]).all(), (name, (err / scale)[normal].max())
         assert (err[~normal] <= 2 * least).all(), name
     assert smallest < 1e-15, smallest
+
+
+@pytest.mark.parametrize("beta,least", [(1e-12, 1e-290), (1e-40, 1e-260), (-1e-60, 1e-240),
+                                        (1e-120, 1e-180), (1e-149, 1e-151)])
+def test_tiny_angles(s2b, beta, least):
+    """d^l_{m,l} for angles whose step factors reach 2^500: sin(beta/2)^(l-m) down to the limit
+    2^(-1021 + bits) of the walk, bits = log2(2 sqrt(2L) cot(beta/2)) rounded up (about `least`)."""
+    L = 65
+    sign, e = top_column(L, beta)
+    with np.errstate(under="ignore"):
+        ref = sign * np.exp(e)
+    flm = np.zeros((L, 2 * L - 1), complex)
+    flm[np.arange(L), L - 1 + np.arange(L)] = 1
+    r = s2b.rotation.rotate_flms(flm, L, (0.0, beta, 0.0))
+    normal = (abs(ref) > least) & (sign != 0)
+    assert np.count_nonzero(normal) >= 2 * L - 1
+    err = abs(r - ref)
+    assert (err[normal] <= 1e-15 * L * abs(ref[normal])).all(), (err / abs(ref))[normal].max()
+    assert (err[~normal] <= 2 * least).all()
+
+
+@pytest.mark.parametrize("L", [1, 2, 65, 130])
+@pytest.mark.parametrize("beta", [0.0, 1e-155, 1e-300])
+def test_identity_leaves_zeros(s2b, rng, L, beta):
+    """No rotation: zeros stay zeros, and the coefficients themselves to rounding."""
+    flm = np.zeros((L, 2 * L - 1), complex)
+    flm[np.arange(L), L - 1 + np.arange(L) // 2] = rng.standard_normal(L) + 1j
+    r = s2b.rotation.rotate_flms(flm, L, (0.0, beta, 0.0))
+    assert (r[flm == 0] == 0).all()
+    assert np.abs(r - flm).max() <= 1e-15 * L * np.abs(flm).max()
