@@ -1020,10 +1020,11 @@ static int build_plan(s2b_plan* p) {
       if (p->M1 != Mr) p->col_f1 = fb.add_bluestein(n1, Mr, n1);
       if (p->col_pruned) p->col_f2 = fb.add_bluestein(n2, Mr, 2 * L);
     }
-    // MW with L a power of two: the passes with the engine's twiddles, whose error they would
-    // exceed otherwise (float, L = 64 and 128: 4.1e-7 and 4.2e-7 against 3.5e-7 and 3.7e-7, with
-    // them 3.3e-7 and 3.6e-7; time 30 and 41 us, on the engine 48 at L = 128)
-    p->col_table_tw = !p->Mreg && p->fwd_mode == 1 && !p->col_pruned && L < 192;
+    // MW with L a power of two, float: the passes with the engine's twiddles, whose error they
+    // would exceed otherwise (L = 64 and 128: 4.1e-7 and 4.2e-7 against 3.5e-7 and 3.7e-7, with
+    // them 3.3e-7 and 3.6e-7; time 30 and 41 us, on the engine 48 at L = 128). In double it does
+    // not show (L = 128 inverse and forward 6.0e-14 either way, 72.0 and 72.7 us).
+    p->col_table_tw = !p->fp64 && !p->Mreg && p->fwd_mode == 1 && !p->col_pruned && L < 192;
   }
   p->maxM = 2;
   if (d.sampling == S2B_HEALPIX) {

@@ -881,8 +881,10 @@ cudaError_t launch_mw_cols(const ColsParams<Real>& p, int ncm, int batch, int M1
   }
   // one DFT buffer plus the 2L bins carried between the two transforms
   const size_t smem = (size_t)(padded_len(M1 > M2 ? M1 : M2) + 2 * p.L) * sizeof(R2);
-  return launch_fft_kernel<Real>(p.table_tw ? mw_cols_kernel<Real, true> : mw_cols_kernel<Real, false>,
-                                 grid, fft_threads(M1 > M2 ? M1 : M2), smem, p, s);
+  auto kern = mw_cols_kernel<Real, false>;
+  if constexpr (sizeof(Real) == 4)
+    if (p.table_tw) kern = mw_cols_kernel<Real, true>;
+  return launch_fft_kernel<Real>(kern, grid, fft_threads(M1 > M2 ? M1 : M2), smem, p, s);
 }
 
 template <typename Real>
