@@ -1152,19 +1152,22 @@ enum FwChain { kFwRowsInv, kFwRowsFwd, kFwColsInv, kFwColsFwd };
 //   rows inverse    float L = 64 6.3 -> 7.7, 128 11.9 -> 13.5, 129 23.1 -> 16.8; double 64 7.3 -> 9.4,
 //                   96 13.0 -> 13.6, 128 19.8 -> 17.3, 129 30.7 -> 24.4; powers of two (MWSS): float
 //                   L = 128 7.3 -> 5.6, double 128 7.8 -> 8.0, 256 25.3 -> 16.2
-//   rows forward    float L = 64 6.5 -> 6.1, 128 12.3 -> 11.9; double 64 7.4 -> 7.5, 65 10.6 -> 9.4;
-//                   powers of two: float L = 128 7.2 -> 5.3, double 128 7.9 -> 8.3, 256 23.5 -> 16.3
+//   rows forward    float L = 64 6.5 -> 6.1, 128 12.3 -> 11.9 (from a flushed L2 the pair of calls
+//                   251 -> 255), 129 23.7 -> 15.9; double 64 7.4 -> 7.5, 65 10.6 -> 9.4; powers of two:
+//                   float L = 128 7.2 -> 5.3, double 128 7.9 -> 8.3, 256 23.5 -> 16.3
 //   columns inverse float L = 128 21.6 -> 28.2, 129 42.2 -> 31.3; double 96 23.7 -> 24.6, 129 56.0 ->
 //                   43.7; powers of two: float L = 256 34.1 -> 49.8, 512 (N = 3) 55.0 -> 43.8
 //   columns forward float L = 128 40.8 -> 43.1, 129 90.9 -> 72.9; double 64 19.5 -> 25.9, 65 38.7 ->
 //                   29.6; powers of two: float L = 256 127 -> 145, 512 (N = 3) 214 -> 191
-// L = 128 in all, inverse + forward: float 231 us, 242 with the engine from 256 points on.
+// L = 128 in all, inverse + forward: float 231 us, 242 with the engine from 256 points on. From a
+// flushed L2 the engine's further tables count: double columns forward on 512 points then gain
+// nothing on average (whole forward L = 65 117 -> 109 us, 96 147 -> 153, 128 197 -> 195).
 template <typename Real>
 constexpr int fw_reg_from(FwChain c, bool blu) {
   constexpr bool f32 = sizeof(Real) == 4;
   switch (c) {
     case kFwRowsInv: return blu ? 10 : f32 ? 8 : 9;
-    case kFwRowsFwd: return blu || f32 ? 8 : 9;
+    case kFwRowsFwd: return !f32 ? 9 : blu ? 10 : 8;
     case kFwColsInv: return 10;
     default: return !blu ? 11 : f32 ? 10 : 9;
   }
