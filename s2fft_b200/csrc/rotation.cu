@@ -600,10 +600,12 @@ constexpr int kWalkThreads = 128;  // also the steps of a staged chunk
 // 43 / 38 us against 39 / 33, whose warps reach the plain loop earlier; L = 1024 620 / 589
 // against 619 / 603; L = 2048 4157 / 4042 against 4248 / 4165.)
 // A non-finite coefficient makes its degree NaN, as a product with a zero would.
-// Grid: (order tiles, degrees from the largest, maps). Bound by the FP64 pipe (six operations
-// per value) and the shared-memory broadcasts (48 bytes per step for the R orders of a lane),
-// with no reduction across lanes: L = 1024, one float64 map, 0.49-0.63 ms over beta (2.6-3.3 ms
-// with recurrences along the degree, whose sums over n crossed lanes, warps and a cluster).
+// Grid: (order tiles, degrees from the largest, maps). Six FP64 operations per value and 48 bytes
+// of shared-memory broadcasts per step for the R orders of a lane, with no reduction across lanes:
+// L = 1024, one float64 map, 0.48-0.62 ms over beta (2.6-3.3 ms with recurrences along the degree,
+// whose sums over n crossed lanes, warps and a cluster). ncu there at beta = 1.9: FP64 pipe 53 %,
+// shared-memory pipe 52 %, issue 45 %; the barriers between chunks are the first stall, as the
+// walks of a CTA end at different steps.
 template <typename R2, int R, int G>
 __global__ void __launch_bounds__(kWalkThreads, 4) rotate_walk_kernel(RotParams p) {
   // two staged chunks: (A, C) of each step, then its two weights; at the end the exchange

@@ -87,13 +87,6 @@ __device__ __forceinline__ void reg_stage(R2* x, const R2 (&bp)[NS], bool inv) {
   }
 }
 
-// NS fused radix-2 stages on the 2^NS points x[ST * a] (a < 2^NS) of one group whose base
-// point is r modulo its smallest span q. tws[k * stride] = b^(2^k), k < NS, with
-// b = exp(-2 pi i r 2^sh / M), sh = log2(M / (2^NS q)) (conjugated when inv): the twiddles
-// of the group, read from the register-engine table (FFTDesc::rtw_off), where consecutive
-// threads read consecutive entries. DIF: spans decreasing; DIT: increasing. The stage of
-// span s q pairs points s apart and multiplies by b^(2^NS / (2 s)) exp(-i pi k / s), k the
-// position within the pair block (the derivation of fft_pass in s2b_fft_dev.h).
 // the twiddles b^(2^k) = tws[k * stride], k < NS, of one group (conjugated when inv)
 template <int NS, typename R2>
 __device__ __forceinline__ void reg_twiddles(R2 (&bp)[NS], const R2* __restrict__ tws, int stride,
