@@ -95,8 +95,7 @@ struct Inv2Layout {
   // (VST: staged by bulk copy; otherwise each lane reads its own from global memory, which
   // leaves room for one more CTA per SM)
   static constexpr size_t v_bytes = VST ? (size_t)2 * NRT * kFwdBlock * 2 * sizeof(Real) : 0;
-  static constexpr size_t row_bytes = 2 * NRT * sizeof(int);  // ftm rows of the rings, mirrors
-  static constexpr size_t fixed_bytes = 2 * stage_bytes + v_bytes + 32 + row_bytes;
+  static constexpr size_t fixed_bytes = 2 * stage_bytes + v_bytes + 32;
   static constexpr int NBUF =
       3 * (fixed_bytes + 2 * buf_elems * sizeof(Piece) + 1024) <= 228 * 1024 ? 2 : 1;
   static constexpr size_t buf_bytes = (size_t)NBUF * buf_elems * sizeof(Piece);
@@ -272,12 +271,20 @@ __device__ __forceinline__ bool lat_inv2_tile(const Inv2Params& p, int bx, int b
     lmax = kb1 * kFwdBlock + kFwdBlock - 1;
   if (lmax > L - 1) lmax = L - 1;
 
-  // ftm rows of the tile's rings (and, symmetric, of their mirrors: none for the equator)
-  int* const rowS = reinterpret_cast<int*>(mbar + 4);
-  for (int i = tid; i < NRT; i += NT) {
-    const int r = r0 + i;
-    rowS[i] = r < p.nrings ? p.ring_row[r] : -1;
-    rowS[NRT + i] = SYM && r < p.nrings && RS - 1 - r != r ? p.ring_row[RS - 1 - r] : -1;
+  // the reduction gives a thread order S = tid % R of a group and NK rings: their ftm rows (and,
+  // symmetric, their mirrors': none for the equator), looked up once
+  constexpr int NK = R * NRT / NT;
+  static_assert(R * NRT % NT == 0 && NT % R == 0, "whole passes of the reduction");
+  R2* frow[NK];
+  R2* fmir[SYM ? NK : 1] = {};
+#pragma unroll
+  for (int k = 0; k < NK; ++k) {
+    const int pos = tid / R + k * (NT / R), r = r0 + (pos % 32) * T + pos / 32;
+    R2* const ftm = reinterpret_cast<R2*>(p.ftm) + (size_t)b * p.nrows * p.ncol;
+    frow[k] = r < p.nrings ? ftm + (size_t)p.ring_row[r] * p.ncol : nullptr;
+    if constexpr (SYM)
+      if (r < p.nrings && RS - 1 - r != r)
+        fmir[k] = ftm + (size_t)p.ring_row[RS - 1 - r] * p.ncol;
   }
   // start values read from global memory: each lane's line is prefetched into L1 one group
   // before the group that starts the state (a group is thousands of cycles of FMAs)
@@ -391,30 +398,30 @@ __device__ __forceinline__ bool lat_inv2_tile(const Inv2Params& p, int bx, int b
     // warps' partial sums -> ring spectra. The R orders of a ring are neighbours in its
     // spectrum, so they go to neighbouring lanes: a warp's atomics cover 32 / R rows in runs
     // of R entries instead of 32 rows.
-    for (int it = tid; it < R * NRT; it += NT) {
-      const int S = it % R, pos = it / R, rr = (pos % 32) * T + pos / 32;
-      const int m = mgrp - S, row = rowS[rr];
-      if (m < p.mlo || m > lmax || row < 0) continue;
-      const Piece* const e = buf + S * Lay::step_elems + pos;
-      Acc s = Lay::get(e);
+    const int m = mgrp - tid % R;
+    if (m >= p.mlo && m <= lmax) {
 #pragma unroll
-      for (int x = 1; x < W; ++x) acc_add(s, Lay::get(e + x * NRT));
-      R2* const ftm = reinterpret_cast<R2*>(p.ftm) + (size_t)b * p.nrows * p.ncol;
-      if constexpr (SYM) {
-        // ring r gets E + O, its mirror E - O (the equator, its own mirror, E + O once)
-        const Piece* const eo = e + Lay::NP * Lay::piece_elems;
-        Acc o = Lay::get(eo);
+      for (int k = 0; k < NK; ++k) {
+        if (!frow[k]) continue;
+        const Piece* const e = buf + (tid % R) * Lay::step_elems + tid / R + k * (NT / R);
+        Acc s = Lay::get(e);
 #pragma unroll
-        for (int x = 1; x < W; ++x) acc_add(o, Lay::get(eo + x * NRT));
-        const int mirror = rowS[NRT + rr];
-        if (mirror >= 0) {
-          Acc d = s;
-          acc_fma(d, Real(-1), o);
-          inv2_store<DUAL>(ftm + (size_t)mirror * p.ncol, d, L, m, p.mo, half);
+        for (int x = 1; x < W; ++x) acc_add(s, Lay::get(e + x * NRT));
+        if constexpr (SYM) {
+          // ring r gets E + O, its mirror E - O (the equator, its own mirror, E + O once)
+          const Piece* const eo = e + Lay::NP * Lay::piece_elems;
+          Acc o = Lay::get(eo);
+#pragma unroll
+          for (int x = 1; x < W; ++x) acc_add(o, Lay::get(eo + x * NRT));
+          if (fmir[k]) {
+            Acc d = s;
+            acc_fma(d, Real(-1), o);
+            inv2_store<DUAL>(fmir[k], d, L, m, p.mo, half);
+          }
+          acc_add(s, o);
         }
-        acc_add(s, o);
+        inv2_store<DUAL>(frow[k], s, L, m, p.mo, half);
       }
-      inv2_store<DUAL>(ftm + (size_t)row * p.ncol, s, L, m, p.mo, half);
     }
     if constexpr (Lay::NBUF == 1) __syncthreads();  // buf is rewritten by the next group
   }
