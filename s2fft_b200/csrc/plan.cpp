@@ -923,18 +923,13 @@ static int build_plan(s2b_plan* p) {
     // launch shape of the inverse kernel, measured at L = 256 ... 1024 (MW, HEALPix; float):
     // eight segments along m (against four: 10-11 % faster at L = 256 and 512 with the
     // tiles below, 1 % at 1024), start values read from global memory (shared memory for 3
-    // CTAs per SM), two rings per lane in float from L = 512 and one below; in double two from
-    // L = 400 at spin 0 (66 us against 69, L = 1024 451 against 531), 250 otherwise (L = 200 36
-    // against 33, L = 256 38 against 45)
+    // CTAs per SM), two rings per lane in float from L = 512 and one below (MW spin 0 L = 400 53 us
+    // against 48, 512 61 against 70; spin 2 GL 512 88.4 against 91.1, 640 144.3 and 144.2, 1024 381 and
+    // 385, DH 1024 668 and 678, 1500 1926 and 1973); in double two from L = 400 at spin 0 (65.4 against
+    // 68.2, L = 300 50 against 47), 250 otherwise (L = 200 36 against 33, 250 38.5 against 45, 300 60
+    // against 59, 400 85 against 89)
     p->inv_nseg = kInvSegMax;
-    if (p->fp64)
-      p->tile_inv = L >= (d.spin != 0 ? 250 : 400) ? 2 : 3;
-    else
-      // (spin != 0: one again from L = 640, with about two rings per degree, DH and HEALPix, from
-      // 1024; spin 2, us, two -> one ring per lane: GL L = 640 147.5 -> 146.4, 800 235.2 -> 232.0, 1400
-      // 941 -> 925; DH 640 243.2 -> 246.5, 800 391.4 -> 393.5, 1024 702.0 -> 698.0, 1400 1733 -> 1724)
-      p->tile_inv =
-          L >= 512 && (d.spin == 0 || L < (p->inv_nrings > L + 1 ? 1024 : 640)) ? 2 : 3;
+    p->tile_inv = L >= (!p->fp64 ? 512 : d.spin != 0 ? 250 : 400) ? 2 : 3;
     // symmetric inverse: one ring pair per lane (two would double the partial sums in
     // shared memory and drop to 2 CTAs per SM; measured slower at L = 256 ... 2048)
     if (p->inv_sym) p->tile_inv = 3;
@@ -1568,10 +1563,10 @@ static int run_forward_adjoint(s2b_plan* p, const void* gflm, void* gf, char* ws
   lp.mlo = lowm_orders(p);
   // One ring per lane, start values staged: without segments along m there are few CTAs, and two
   // rings per lane halve them (and staged in double leave one CTA per SM): MW, us, two rings and
-  // staged -> this: double L = 64 / 256 / 1024 spin 0 64 / 156 / 1466 -> 51 / 126 / 1311, spin 2
-  // 60 / 145 / 1891 -> 53 / 129 / 1650; float spin 0 53 / 125 / 830 -> 43 / 94 / 760, spin 2
-  // 53 / 151 -> 47 / 111. Float with spin from L = 624 on: start values from global memory (L = 608
-  // staged 460 against 468, 640 501 against 484, 1024 933 against 899).
+  // staged -> this: double L = 64 / 256 / 1024 spin 0 64 / 156 / 1466 -> 51 / 123 / 1285, spin 2
+  // 60 / 145 / 1891 -> 51 / 126 / 1606; float spin 0 53 / 125 / 830 -> 43 / 93 / 749, spin 2
+  // 53 / 151 / 909 -> 47 / 109 / 875. Float with spin from L = 624 on: start values from global memory
+  // (L = 608 staged 450 against 461, 640 491 against 478, 700 577 against 557).
   lp.tile = !p->fp64 && d.spin != 0 && L >= 624 ? 3 : 1;
   S2B_CK(launch_inv2(p->fp64, p->dual, lp, s));
   if (int rc_ = run_lowm_synth(p, lp, p->fwd_rings, s)) return rc_;
